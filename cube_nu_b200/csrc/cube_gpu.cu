@@ -1472,8 +1472,9 @@ static int enqueue_kick_a(cube_ctx* c) {
   // PM3 mass over the boxes' physical cells, from the classes just found
   if (c->P.pm3_on) {
     unsigned long long* ms3 = c->msum + 2 * MASS_SLOTS * MASS_STRIDE;
-    if (fixed) LAUNCH(c, K_MASS, 1, k_mass_pm3<true><<<nblk(G.ncells), 256, 0, c->s>>>(G, c->cstart, c->xp, c->ires, ms3));
-    else LAUNCH(c, K_MASS, 1, k_mass_pm3<false><<<nblk(G.ncells), 256, 0, c->s>>>(G, c->cstart, c->xp, c->ires, ms3));
+    const int gpb = mass3_groups(G.ncells);
+    if (fixed) LAUNCH(c, K_MASS, 1, k_mass_pm3<true><<<nblk(G.ncells, 32 * gpb), MASS3_T, 0, c->s>>>(G, c->cstart, c->xp, c->ires, gpb, ms3));
+    else LAUNCH(c, K_MASS, 1, k_mass_pm3<false><<<nblk(G.ncells, 32 * gpb), MASS3_T, 0, c->s>>>(G, c->cstart, c->xp, c->ires, gpb, ms3));
   }
   return 0;
 }

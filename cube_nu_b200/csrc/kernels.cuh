@@ -770,89 +770,148 @@ __device__ __forceinline__ void mass_box(const Geo& G, int iapm, const double lf
 // direction (-1, 0, +1) of 0-based cell index i relative to the physical range 0..nfp-1
 __device__ __forceinline__ int mass_dir(int i, int nfp) { return i < 0 ? -1 : (i >= nfp ? 1 : 0); }
 
-// The class-boundary part: one thread per coarse cell; a cell in a face layer of its
-// subtile whose neighbour subtile across that face has another class corrects the own-box
-// sums that k_interp_pm3 added for its particles.  Every other cell returns at once.
+// The class-boundary part.  A cell in a face layer of its subtile whose neighbour subtile
+// across that face has another class corrects the own-box sums that k_interp_pm3 added for
+// its particles.  A block looks at gpb groups of 32 consecutive coarse cells, one cell per
+// thread, and its threads then share out the particles of a group's cells to correct (a
+// prefix of the counts and a binary search), so a cell of tens of thousands of particles is
+// not walked by one thread: that made the kernel as long as its fullest boundary cell, 112 ms
+// of a 147 ms kick of 128^3 clustered particles (largest cell 3e4), 0.2 ms now.  A group's
+// sum is added to the mass slots as one value.
+constexpr int MASS3_T = 256;
 template <bool FIXED>
-__global__ void __launch_bounds__(256) k_mass_pm3(Geo G, const int64_t* __restrict__ cstart,
-                                                  const void* __restrict__ xp, const int32_t* __restrict__ ires,
-                                                  void* msum) {
-  const int64_t cell = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(MASS3_T) k_mass_pm3(Geo G, const int64_t* __restrict__ cstart,
+                                                      const void* __restrict__ xp, const int32_t* __restrict__ ires,
+                                                      int gpb, void* msum) {
+  using Acc = typename MassAcc<FIXED>::T;
+  __shared__ unsigned flags[MASS3_T / 32];  // cells to correct, a bit each, per group
+  __shared__ int64_t pre[33];               // prefix of their particle counts
+  __shared__ int32_t list[32];
+  __shared__ Acc part[MASS3_T / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t cell0 = (int64_t)blockIdx.x * gpb * 32;
+  if (wid < gpb) {
+    const int64_t cell = cell0 + threadIdx.x;
+    bool any = false;
+    if (cell < G.ncells && owned_cell(G, cell) && cstart[cell + 1] > cstart[cell]) {
+      int g[3], tc[3][2], uc[3][2], lc[3][2], nca[3];
+      cell_coords(G, cell, g[0], g[1], g[2]);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) nca[d] = sub_cands(G, g[d], tc[d], uc[d], lc[d]);
+      if (nca[0] * nca[1] * nca[2] > 1) {
+        const int t0[3] = {tc[0][0], tc[1][0], tc[2][0]}, u0[3] = {uc[0][0], uc[1][0], uc[2][0]};
+        const int own = ires[subtile_id(G, t0, u0)];
+        for (int cz = 0; cz < nca[2]; ++cz)
+          for (int cy = 0; cy < nca[1]; ++cy)
+            for (int cx = 0; cx < nca[0]; ++cx) {
+              const int t[3] = {tc[0][cx], tc[1][cy], tc[2][cz]}, u[3] = {uc[0][cx], uc[1][cy], uc[2][cz]};
+              any |= ires[subtile_id(G, t, u)] != own;
+            }
+      }
+    }
+    const unsigned bits = __ballot_sync(0xffffffffu, any);
+    if (lane == 0) flags[wid] = bits;
+  }
+  __syncthreads();
+  for (int grp = 0; grp < gpb; ++grp) {
+  const unsigned bits = flags[grp];
+  if (bits == 0) continue;  // block-uniform
+  const int nl = __popc(bits);
+  __syncthreads();  // list, pre and part are free again
+  if (wid == 0) {
+    const bool mine = (bits >> lane) & 1u;
+    const int r = __popc(bits & ((1u << lane) - 1u));
+    const int64_t cell = cell0 + grp * 32 + lane;
+    const int64_t cnt = mine ? cstart[cell + 1] - cstart[cell] : 0;
+    const int64_t incl = warp_incl_scan(cnt);
+    if (mine) {
+      list[r] = (int32_t)cell;
+      pre[r] = incl - cnt;
+    }
+    if (lane == 31) pre[nl] = incl;
+  }
+  __syncthreads();
+  const int64_t total = pre[nl];
   MassAcc<FIXED> mass;
-  int g[3], tc[3][2], uc[3][2], lc[3][2], nca[3] = {1, 1, 1};
-  bool any = false;
-  int own = 0;
-  if (cell < G.ncells && owned_cell(G, cell)) {
-    cell_coords(G, cell, g[0], g[1], g[2]);
+  for (int64_t v = threadIdx.x; v < total; v += MASS3_T) {
+    int lo = 0, hi = nl;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (pre[mid] <= v) lo = mid;
+      else hi = mid;
+    }
+    const int64_t ip = cstart[list[lo]] + (v - pre[lo]);
+    int g[3], tc[3][2], uc[3][2], lc[3][2], nca[3];
+    cell_coords(G, list[lo], g[0], g[1], g[2]);
 #pragma unroll
     for (int d = 0; d < 3; ++d) nca[d] = sub_cands(G, g[d], tc[d], uc[d], lc[d]);
-    if (nca[0] * nca[1] * nca[2] > 1) {
-      const int t0[3] = {tc[0][0], tc[1][0], tc[2][0]}, u0[3] = {uc[0][0], uc[1][0], uc[2][0]};
-      own = ires[subtile_id(G, t0, u0)];
-      for (int cz = 0; cz < nca[2]; ++cz)
-        for (int cy = 0; cy < nca[1]; ++cy)
-          for (int cx = 0; cx < nca[0]; ++cx) {
-            const int t[3] = {tc[0][cx], tc[1][cy], tc[2][cz]}, u[3] = {uc[0][cx], uc[1][cy], uc[2][cz]};
-            any |= ires[subtile_id(G, t, u)] != own;
-          }
-    }
-  }
-  if (any) {
+    const int t0[3] = {tc[0][0], tc[1][0], tc[2][0]}, u0[3] = {uc[0][0], uc[1][0], uc[2][0]};
+    const int own = ires[subtile_id(G, t0, u0)];
     const int nfp0 = G.nfp[own];
-    const int u0[3] = {uc[0][0], uc[1][0], uc[2][0]};
-    for (int64_t ip = cstart[cell]; ip < cstart[cell + 1]; ++ip) {
-      double f[3];
+    double f[3];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) f[d] = zfrac(load_code(xp, G.izipx, 3 * ip + d), G);
-      const double lf0[3] = {(double)lc[0][0] + f[0], (double)lc[1][0] + f[1], (double)lc[2][0] + f[2]};
-      int i2[3];
-      float w[3][3];
-      mass_box<FIXED>(G, own, lf0, u0, i2, w);
-      for (int cz = 0; cz < nca[2]; ++cz)
-        for (int cy = 0; cy < nca[1]; ++cy)
-          for (int cx = 0; cx < nca[0]; ++cx) {
-            if (cx + cy + cz == 0) continue;
-            const int t[3] = {tc[0][cx], tc[1][cy], tc[2][cz]};
-            const int u[3] = {uc[0][cx], uc[1][cy], uc[2][cz]};
-            const int nb = ires[subtile_id(G, t, u)];
-            if (nb == own) continue;
-            int dir[3];
-            const int cc[3] = {cx, cy, cz};
+    for (int d = 0; d < 3; ++d) f[d] = zfrac(load_code(xp, G.izipx, 3 * ip + d), G);
+    const double lf0[3] = {(double)lc[0][0] + f[0], (double)lc[1][0] + f[1], (double)lc[2][0] + f[2]};
+    int i2[3];
+    float w[3][3];
+    mass_box<FIXED>(G, own, lf0, u0, i2, w);
+    for (int cz = 0; cz < nca[2]; ++cz)
+      for (int cy = 0; cy < nca[1]; ++cy)
+        for (int cx = 0; cx < nca[0]; ++cx) {
+          if (cx + cy + cz == 0) continue;
+          const int t[3] = {tc[0][cx], tc[1][cy], tc[2][cz]};
+          const int u[3] = {uc[0][cx], uc[1][cy], uc[2][cz]};
+          const int nb = ires[subtile_id(G, t, u)];
+          if (nb == own) continue;
+          int dir[3];
+          const int cc[3] = {cx, cy, cz};
 #pragma unroll
-            for (int d = 0; d < 3; ++d)  // sub_cands: the first coarse cell of a subtile reaches down, the last up
-              dir[d] = cc[d] == 0 ? 0 : ((lc[d][0] % G.ntt) == 0 ? -1 : 1);
-            // the own contributions in that direction leave the sum ...
-            MassAcc<FIXED> sub;
+          for (int d = 0; d < 3; ++d)  // sub_cands: the first coarse cell of a subtile reaches down, the last up
+            dir[d] = cc[d] == 0 ? 0 : ((lc[d][0] % G.ntt) == 0 ? -1 : 1);
+          // the own contributions in that direction leave the sum ...
+          MassAcc<FIXED> sub;
 #pragma unroll
-            for (int a3 = 0; a3 < 3; ++a3)
+          for (int a3 = 0; a3 < 3; ++a3)
 #pragma unroll
-              for (int a2 = 0; a2 < 3; ++a2)
+            for (int a2 = 0; a2 < 3; ++a2)
 #pragma unroll
-                for (int a1 = 0; a1 < 3; ++a1)
-                  if (mass_dir(i2[0] - 2 + a1, nfp0) == dir[0] && mass_dir(i2[1] - 2 + a2, nfp0) == dir[1] &&
-                      mass_dir(i2[2] - 2 + a3, nfp0) == dir[2])
-                    sub.add(__fmul_rn(__fmul_rn(w[0][a1], w[1][a2]), w[2][a3]));
-            mass.v -= sub.v;
-            // ... and the neighbour's own physical contributions at its class come in
-            const double lf[3] = {(double)lc[0][cx] + f[0], (double)lc[1][cy] + f[1], (double)lc[2][cz] + f[2]};
-            int j2[3];
-            float v[3][3];
-            mass_box<FIXED>(G, nb, lf, u, j2, v);
-            const int nfp = G.nfp[nb];
+              for (int a1 = 0; a1 < 3; ++a1)
+                if (mass_dir(i2[0] - 2 + a1, nfp0) == dir[0] && mass_dir(i2[1] - 2 + a2, nfp0) == dir[1] &&
+                    mass_dir(i2[2] - 2 + a3, nfp0) == dir[2])
+                  sub.add(__fmul_rn(__fmul_rn(w[0][a1], w[1][a2]), w[2][a3]));
+          mass.v -= sub.v;
+          // ... and the neighbour's own physical contributions at its class come in
+          const double lf[3] = {(double)lc[0][cx] + f[0], (double)lc[1][cy] + f[1], (double)lc[2][cz] + f[2]};
+          int j2[3];
+          float v3[3][3];
+          mass_box<FIXED>(G, nb, lf, u, j2, v3);
+          const int nfp = G.nfp[nb];
 #pragma unroll
-            for (int a3 = 0; a3 < 3; ++a3)
+          for (int a3 = 0; a3 < 3; ++a3)
 #pragma unroll
-              for (int a2 = 0; a2 < 3; ++a2)
+            for (int a2 = 0; a2 < 3; ++a2)
 #pragma unroll
-                for (int a1 = 0; a1 < 3; ++a1)
-                  if ((unsigned)(j2[0] - 2 + a1) < (unsigned)nfp && (unsigned)(j2[1] - 2 + a2) < (unsigned)nfp &&
-                      (unsigned)(j2[2] - 2 + a3) < (unsigned)nfp)
-                    mass.add(__fmul_rn(__fmul_rn(v[0][a1], v[1][a2]), v[2][a3]));
-          }
-    }
+              for (int a1 = 0; a1 < 3; ++a1)
+                if ((unsigned)(j2[0] - 2 + a1) < (unsigned)nfp && (unsigned)(j2[1] - 2 + a2) < (unsigned)nfp &&
+                    (unsigned)(j2[2] - 2 + a3) < (unsigned)nfp)
+                  mass.add(__fmul_rn(__fmul_rn(v3[0][a1], v3[1][a2]), v3[2][a3]));
+        }
   }
-  mass.flush(msum);
+  for (int o = 16; o > 0; o >>= 1) mass.v += __shfl_xor_sync(0xffffffffu, mass.v, o);
+  if (lane == 0) part[wid] = mass.v;
+  __syncthreads();
+  if (wid == 0) {
+    MassAcc<FIXED> sum;
+    if (lane < MASS3_T / 32) sum.v = part[lane];
+    sum.flush(msum);
+  }
+  }
 }
+
+// Groups of 32 cells per block of k_mass_pm3: one where the box has few cells (at most 2^18,
+// a few blocks per SM), so that its full cells spread over the SMs; eight (a cell per
+// thread) where most blocks only look.
+inline int mass3_groups(int64_t ncells) { return ncells <= (1 << 18) ? 1 : MASS3_T / 32; }
 
 // Owner-computes form of the fixed-point PM3 deposit: one block per region of
 // DEP3_R x DEP3_R x DEP3_RZ cells of one box.  The block sums, in shared memory, the contributions of the

@@ -1459,7 +1459,7 @@ static int enqueue_kick_a(cube_ctx* c) {
   CK(mark(c, c->ev[2]));
   // ---------------- subtile classes (kick.f90:108-138) ----------------
   CK(cudaMemsetAsync(c->napm, 0, 32, c->s));
-  LAUNCH(c, K_CLASSIFY, 1, k_classify<<<nblk(c->ns3), 256, 0, c->s>>>(G, c->rhoc, c->ns3, c->ires, c->napm));
+  LAUNCH(c, K_CLASSIFY, 1, k_classify<<<(unsigned)c->ns3, CLASSIFY_T, 0, c->s>>>(G, c->rhoc, c->ires, c->napm));
   if (G.nslab > 1) {  // every rank's classes (the PM3 mass needs its neighbours')
     const int rc = comm_allreduce(c, c->ires, c->ns3, CUBE_DT_I32, CUBE_OP_MAX, 1);
     if (rc) return rc;
@@ -1923,7 +1923,7 @@ static int step_graph(cube_ctx* c, const cube_step_in* in, cube_step_out* out) {
   if (rc) return rc;
   if (!c->have_est) {  // first step: classes of the current state
     CK(cudaMemsetAsync(c->napm, 0, 32, c->s));
-    LAUNCH(c, K_CLASSIFY, 1, k_classify<<<nblk(c->ns3), 256, 0, c->s>>>(c->G, c->rhoc, c->ns3, c->ires, c->napm));
+    LAUNCH(c, K_CLASSIFY, 1, k_classify<<<(unsigned)c->ns3, CLASSIFY_T, 0, c->s>>>(c->G, c->rhoc, c->ires, c->napm));
     CK(cudaMemcpyAsync(c->napm_est, c->napm, 32, cudaMemcpyDeviceToHost, c->s));
     CK(cudaStreamSynchronize(c->s));
     c->have_est = true;
@@ -2612,7 +2612,7 @@ int cube_gpu_subtile_class(cube_ctx* c, int32_t* ires, int64_t n) {
   if (!c || !ires || n < c->ns3) return fail(CUBE_E_ARG, "bad argument");
   CK(cudaSetDevice(c->device));
   CK(cudaMemsetAsync(c->napm, 0, 32, c->s));
-  LAUNCH(c, K_CLASSIFY, 1, k_classify<<<nblk(c->ns3), 256, 0, c->s>>>(c->G, c->rhoc, c->ns3, c->ires, c->napm));
+  LAUNCH(c, K_CLASSIFY, 1, k_classify<<<(unsigned)c->ns3, CLASSIFY_T, 0, c->s>>>(c->G, c->rhoc, c->ires, c->napm));
   CK(cudaMemcpyAsync(ires, c->ires, c->ns3 * 4, cudaMemcpyDeviceToHost, c->s));
   CK(cudaStreamSynchronize(c->s));
   return 0;

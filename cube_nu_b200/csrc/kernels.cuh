@@ -1554,25 +1554,33 @@ __global__ void __launch_bounds__(256, 3) k_interp_pm3(Geo G, int64_t np, const 
 // =================================================================================
 // Subtile classes (kick.f90:108-133) and the box slot map of one class.
 // =================================================================================
-__global__ void k_classify(Geo G, const int32_t* __restrict__ rhoc, int ns3, int32_t* __restrict__ ires,
-                           int32_t* __restrict__ napm) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ns3) return;
+// One block per subtile: its threads read the subtile's rows of cells side by side.  (One
+// thread per subtile read ntt^3 counts one after the other: 0.74 ms at ntt = 16, whatever
+// the number of subtiles, against 0.01 ms for 512 of them now.)
+constexpr int CLASSIFY_T = 128;
+__global__ void __launch_bounds__(CLASSIFY_T) k_classify(Geo G, const int32_t* __restrict__ rhoc,
+                                                         int32_t* __restrict__ ires, int32_t* __restrict__ napm) {
+  __shared__ int part[CLASSIFY_T / 32];
+  const int s = blockIdx.x;
   if (s < G.s0 || s >= G.s1) {  // another rank's subtile: its class arrives by a max-reduction
-    ires[s] = 0;
+    if (threadIdx.x == 0) ires[s] = 0;
     return;
   }
-  const int nns3 = G.nns * G.nns * G.nns;
+  const int nns3 = G.nns * G.nns * G.nns, ntt = G.ntt, nt = G.nt;
   const int T = s / nns3, f = s - T * nns3;
-  const int tx = T % G.nnt, ty = (T / G.nnt) % G.nnt, tz = T / (G.nnt * G.nnt);
   const int ux = f % G.nns, uy = (f / G.nns) % G.nns, uz = f / (G.nns * G.nns);
+  // first cell of the subtile; a tile's cells are stored together, x fastest
+  const int32_t* base = rhoc + (int64_t)T * nt * nt * nt + ((int64_t)uz * ntt * nt + (int64_t)uy * ntt) * nt + ux * ntt;
   int mx = 0;
-  for (int k = 0; k < G.ntt; ++k)
-    for (int j = 0; j < G.ntt; ++j)
-      for (int i = 0; i < G.ntt; ++i) {
-        const int64_t c = cell_index(G, tx * G.nt + ux * G.ntt + i, ty * G.nt + uy * G.ntt + j, tz * G.nt + uz * G.ntt + k);
-        mx = max(mx, rhoc[c]);
-      }
+  for (int c = threadIdx.x; c < ntt * ntt * ntt; c += CLASSIFY_T) {
+    const int row = c / ntt, i = c - row * ntt, k = row / ntt, j = row - k * ntt;
+    mx = max(mx, base[((int64_t)k * nt + j) * nt + i]);
+  }
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < CLASSIFY_T / 32; ++w) mx = max(mx, part[w]);
   const float npc = (float)mx / 64.f;
   const int r = (npc < 24.f) ? 2 : (npc < 114.f) ? 3 : (npc < 320.f) ? 4 : 5;
   ires[s] = r;

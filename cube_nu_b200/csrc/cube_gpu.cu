@@ -513,11 +513,11 @@ void fft2_run(cube_ctx* c, int64_t nbox, const void* real_in, bool fixed, float 
       const unsigned planes = (unsigned)(nbox * N);
       if (fixed) {
         smem_optin(f2::k_fxy3_r2c<N, R1, R2, long long>, smf);
-        LAUNCH(c, kx, 1, f2::k_fxy3_r2c<N, R1, R2, long long><<<planes, f2::PLANE3_THREADS, smf, c->s>>>(
+        LAUNCH(c, kx, 1, f2::k_fxy3_r2c<N, R1, R2, long long><<<planes, f2::PlaneShape<N, R1, R2>::THREADS, smf, c->s>>>(
                              (const long long*)real_in, ck, tw, scale, pt.pr, pt.pc, pt.plr, pt.plc));
       } else {
         smem_optin(f2::k_fxy3_r2c<N, R1, R2, float>, smf);
-        LAUNCH(c, kx, 1, f2::k_fxy3_r2c<N, R1, R2, float><<<planes, f2::PLANE3_THREADS, smf, c->s>>>(
+        LAUNCH(c, kx, 1, f2::k_fxy3_r2c<N, R1, R2, float><<<planes, f2::PlaneShape<N, R1, R2>::THREADS, smf, c->s>>>(
                              (const float*)real_in, ck, tw, scale, pt.pr, pt.pc, pt.plr, pt.plc));
       }
       // plane sizes: the block-per-line column pass hides latency with more warps
@@ -525,7 +525,7 @@ void fft2_run(cube_ctx* c, int64_t nbox, const void* real_in, bool fixed, float 
       smem_optin(f2::k_fcol3<N, R1, R2, 2, 2>, smg);
       LAUNCH(c, kz, 1, f2::k_fcol3<N, R1, R2, 2, 2><<<gc, W * T, smg, c->s>>>(ck, green, tw, W, pt.pc, pt.plc));
       smem_optin(f2::k_fyx3_c2r<N, R1, R2>, smi);
-      LAUNCH(c, kc, 1, f2::k_fyx3_c2r<N, R1, R2><<<planes, f2::PLANE3_THREADS, smi, c->s>>>(
+      LAUNCH(c, kc, 1, f2::k_fyx3_c2r<N, R1, R2><<<planes, f2::PlaneShape<N, R1, R2>::THREADS, smi, c->s>>>(
                            ck, phi_out, tw, inv, pt.pc, pt.pf, pt.plc, pt.plf));
       return;
     }
@@ -603,7 +603,7 @@ void fft2_forward(cube_ctx* c, float* real, const Pitch& pt, int cls) {
     if (fused_layout(c, N)) {
       const size_t smf = f2::Plane3Sm<N>::FWD;
       smem_optin(f2::k_fxy3_r2c<N, R1, R2, float>, smf);
-      LAUNCH(c, cls, 1, f2::k_fxy3_r2c<N, R1, R2, float><<<(unsigned)N, f2::PLANE3_THREADS, smf, c->s>>>(
+      LAUNCH(c, cls, 1, f2::k_fxy3_r2c<N, R1, R2, float><<<(unsigned)N, f2::PlaneShape<N, R1, R2>::THREADS, smf, c->s>>>(
                             real, ck, tw, 1.f, pt.pr, pt.pc, pt.plr, pt.plc));
       LAUNCH(c, cls, 1, f2::k_fcol3<N, R1, R2, 2, 0><<<gc, W * T, smc, c->s>>>(ck, nullptr, tw, W, pt.pc, pt.plc));
       return;

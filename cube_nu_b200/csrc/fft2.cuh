@@ -521,14 +521,28 @@ __global__ void __launch_bounds__(256) k_fx_c2r(const float2* c, float* r, int64
 
 // ---------------------------------------------------------------------------------
 // Plane kernels with register-resident sequences (N <= 144, T = max(R1,R2) <= 16).
-// Rows run warp-synchronously: each warp holds two sequences (lanes 0..T-1 and
-// 16..16+T-1), loads them straight from global memory and exchanges through a skewed
+// Rows run warp-synchronously: each warp holds 32/L sequences (T of L lanes each), loads
+// them straight from global memory and exchanges through a skewed
 // slot layout (slot(k1, n2) = k1*R2 + (n2 + k1) mod R2) that is free of bank conflicts
 // in both directions.  Columns run as in k_fcol3, W columns by T threads per round.
 // The r2c unpack and the c2r Hermitian pack happen on the fly inside the other phase,
 // and column results go straight to global memory.
 // ---------------------------------------------------------------------------------
-constexpr int PLANE3_THREADS = 448;
+// Launch shape of the plane kernels for one N.  A sequence takes T = max(R1, R2) threads; a
+// round of the column phase runs W columns, the fewest equal rounds that fit 448 threads, and
+// the block has just the threads of one round.  The row phase gives a sequence L = 4, 8 or 16
+// lanes, the smallest that hold T, so a warp runs 32/L of them.  Blocks per SM: about 900
+// threads for N >= 96, whose 12- and 16-point DFTs want 72 registers, and up to 1300 for the
+// smaller ones, which are bound by latency (N = 48, 4096 boxes, both passes: 5.2 ms with 448
+// threads and 16 lanes a sequence, two blocks per SM).
+template <int N, int R1, int R2>
+struct PlaneShape {
+  static constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1;
+  static constexpr int L = T <= 4 ? 4 : T <= 8 ? 8 : 16;
+  static constexpr int ROUNDS = (NH * T + 447) / 448, W = (NH + ROUNDS - 1) / ROUNDS;
+  static constexpr int THREADS = (W * T + 31) / 32 * 32;
+  static constexpr int MINB = N == 96 ? 3 : N >= 96 ? 2 : N >= 64 ? 4 : N >= 48 ? 6 : 8;
+};
 
 template <int N>
 struct Plane3Sm {
@@ -548,7 +562,7 @@ __device__ __forceinline__ int skew(int k1, int n2) {
 }
 
 template <int N, int R1, int R2, typename IN>
-__global__ void __launch_bounds__(PLANE3_THREADS, 2) k_fxy3_r2c(const IN* __restrict__ r, float2* __restrict__ c,
+__global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, R1, R2>::MINB) k_fxy3_r2c(const IN* __restrict__ r, float2* __restrict__ c,
                                                                const float2* __restrict__ gtw, float scale, int pr,
                                                                int pc, int64_t plr, int64_t plc) {
   constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1, NP = N / 2;
@@ -562,9 +576,10 @@ __global__ void __launch_bounds__(PLANE3_THREADS, 2) k_fxy3_r2c(const IN* __rest
   float2* cp = c + plane * plc;
   __syncthreads();
   {  // ---- rows: packed pairs (2p, 2p+1) as re/im ----
-    const int lane = threadIdx.x & 31, t = lane & 15;
-    const int g = (threadIdx.x >> 5) * 2 + (lane >> 4);
-    const int ngr = (blockDim.x >> 5) * 2;
+    constexpr int L = PlaneShape<N, R1, R2>::L;
+    const int lane = threadIdx.x & 31, t = lane % L;
+    const int g = (threadIdx.x >> 5) * (32 / L) + lane / L;
+    constexpr int ngr = PlaneShape<N, R1, R2>::THREADS / L;
     for (int p0 = 0; p0 < NP; p0 += ngr) {
       const int p = p0 + g;
       const bool act = p < NP;
@@ -606,7 +621,7 @@ __global__ void __launch_bounds__(PLANE3_THREADS, 2) k_fxy3_r2c(const IN* __rest
   }
   __syncthreads();
   {  // ---- columns kx of the half spectrum, unpacked on the fly ----
-    const int W = (NH < (int)blockDim.x / T) ? NH : (int)blockDim.x / T;
+    constexpr int W = PlaneShape<N, R1, R2>::W;
     const int col = threadIdx.x % W, t = threadIdx.x / W;
     for (int kx0 = 0; kx0 < NH; kx0 += W) {
       const int kx = kx0 + col;
@@ -662,7 +677,7 @@ __global__ void __launch_bounds__(PLANE3_THREADS, 2) k_fxy3_r2c(const IN* __rest
 }
 
 template <int N, int R1, int R2>
-__global__ void __launch_bounds__(PLANE3_THREADS, 2) k_fyx3_c2r(const float2* __restrict__ c, float* __restrict__ r,
+__global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, R1, R2>::MINB) k_fyx3_c2r(const float2* __restrict__ c, float* __restrict__ r,
                                                                const float2* __restrict__ gtw, float inv,
                                                                int pc, int pf, int64_t plc, int64_t plf) {
   constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1, NP = N / 2;
@@ -676,7 +691,7 @@ __global__ void __launch_bounds__(PLANE3_THREADS, 2) k_fyx3_c2r(const float2* __
   float* rp = r + plane * plf;
   __syncthreads();
   {  // ---- inverse y transforms of the columns kx, n = R2*n1 + n2 ----
-    const int W = (NH < (int)blockDim.x / T) ? NH : (int)blockDim.x / T;
+    constexpr int W = PlaneShape<N, R1, R2>::W;
     const int col = threadIdx.x % W, t = threadIdx.x / W;
     for (int kx0 = 0; kx0 < NH; kx0 += W) {
       const int kx = kx0 + col;
@@ -706,9 +721,10 @@ __global__ void __launch_bounds__(PLANE3_THREADS, 2) k_fyx3_c2r(const float2* __
   }
   __syncthreads();
   {  // ---- rows: pack (2p, 2p+1) over the Hermitian extension, inverse x transform ----
-    const int lane = threadIdx.x & 31, t = lane & 15;
-    const int g = (threadIdx.x >> 5) * 2 + (lane >> 4);
-    const int ngr = (blockDim.x >> 5) * 2;
+    constexpr int L = PlaneShape<N, R1, R2>::L;
+    const int lane = threadIdx.x & 31, t = lane % L;
+    const int g = (threadIdx.x >> 5) * (32 / L) + lane / L;
+    constexpr int ngr = PlaneShape<N, R1, R2>::THREADS / L;
     for (int p0 = 0; p0 < NP; p0 += ngr) {
       const int p = p0 + g;
       const bool act = p < NP;

@@ -1731,12 +1731,13 @@ static void enqueue_pp_and_momentum(cube_ctx* c, const unsigned* abort, const PP
     // FP32 candidate positions are exact when lq + offset fits 24 bits: int8 codes, or
     // int16 codes with tile-local coordinates |lq| <= nt < 128
     const bool pp_fast = G.izipx == 1 || G.nt < 127;
-    if (pp_fast)
-      LAUNCH(c, K_PP, 1, k_pp<true><<<nblk(np, 128), 128, 0, c->s>>>(G, np, c->xp, c->pcell, c->cstart, c->ires, c->vp,
-                                                                    c->sd, f2 + 3, vm + 6, c->pairs, c->pairs + 1, abort));
-    else
-      LAUNCH(c, K_PP, 1, k_pp<false><<<nblk(np, 128), 128, 0, c->s>>>(G, np, c->xp, c->pcell, c->cstart, c->ires, c->vp,
-                                                                     c->sd, f2 + 3, vm + 6, c->pairs, c->pairs + 1, abort));
+    auto pp = [&](auto kernel, auto* codes) {
+      LAUNCH(c, K_PP, 1, kernel<<<nblk(np, PP_T), PP_T, 0, c->s>>>(G, np, codes, c->pcell, c->cstart, c->ires, c->vp, c->sd,
+                                                                   f2 + 3, vm + 6, c->pairs, c->pairs + 1, abort));
+    };
+    if (G.izipx == 1) pp(k_pp<true, uint8_t>, static_cast<const uint8_t*>(c->xp));
+    else if (pp_fast) pp(k_pp<true, uint16_t>, static_cast<const uint16_t*>(c->xp));
+    else pp(k_pp<false, uint16_t>, static_cast<const uint16_t*>(c->xp));
   }
   mark(c, c->ev[4]);
   const int64_t o = G.nslab > 1 ? c->own0 : 0, npo = G.nslab > 1 ? c->own1 - c->own0 : np;

@@ -1648,121 +1648,219 @@ __global__ void __launch_bounds__(1024) k_build_lists(const int32_t* __restrict_
 // coarse cells its range can reach; equivalent to the reference's PP-cell lists
 // (the PP cell 4/rsf fine cells is wider than the range 3.5/rsf).
 // =================================================================================
-// The softened force law's coefficient (1/35)/apm^2, a constant of apm.
-__device__ __forceinline__ float F_ra_coef(float apm) { return __fdiv_rn(__fdiv_rn(1.f, 35.f), __fmul_rn(apm, apm)); }
-
-// F_ra with its coefficient c = F_ra_coef(apm) passed in, for callers that evaluate it for
-// one apm many times; the same operations as F_ra.
-__device__ __forceinline__ float F_ra_c(float r, float apm, float c) {
-  const float ep = __fdiv_rn(2.f * r, apm);
-  if (apm == 0.f || ep > 2.f) return __fdiv_rn(1.f, __fmul_rn(r, r));
-  const float e2 = ep * ep, e3 = e2 * ep, e4 = e3 * ep, e5 = e4 * ep, e6 = e5 * ep;
-  if (ep > 1.f) return c * (12.f * (1.f / e2) - 224.f + 896.f * ep - 840.f * e2 + 224.f * e3 + 70.f * e4 - 48.f * e5 + 7.f * e6);
-  if (ep > 0.f) return c * (224.f * ep - 224.f * e3 + 70.f * e4 + 48.f * e5 - 21.f * e6);
-  return 0.f;
-}
-
-__device__ __forceinline__ float F_ra(float r, float apm) {
-  const float ep = __fdiv_rn(2.f * r, apm);
-  if (apm == 0.f || ep > 2.f) return __fdiv_rn(1.f, __fmul_rn(r, r));
-  return F_ra_c(r, apm, F_ra_coef(apm));
+// F_ra of kick.f90 at r = e * apm / 2 <= apm, from e, apm's coefficient c = (1/35)/apm^2 and
+// 12/e^2 (the S2 cloud's force; 1/r^2 beyond).
+// Rounded step by step (no contraction), so that every kernel gives the same bits.
+__device__ __forceinline__ float F_s2(float e, float c, float twelve_over_e2) {
+  const float e2 = __fmul_rn(e, e);
+  const float near = __fmul_rn(
+      e, __fmaf_rn(e2, __fmaf_rn(e, __fmaf_rn(e, __fmaf_rn(e, -21.f, 48.f), 70.f), -224.f), 224.f));
+  const float poly = __fmaf_rn(
+      e, __fmaf_rn(e, __fmaf_rn(e, __fmaf_rn(e, __fmaf_rn(e, __fmaf_rn(e, 7.f, -48.f), 70.f), 224.f), -840.f), 896.f), -224.f);
+  return __fmul_rn(c, e > 1.f ? __fadd_rn(poly, twelve_over_e2) : near);
 }
 
 // Candidate coordinate (xq in kick.f90:424): ((lq + (u+0.5)*x_res) * ratio_cs) rounded to
 // float.  FAST: lq + (u+0.5)*x_res has at most 8*izipx+1+log2|lq| significant bits; when
-// that is <= 24 (int8 codes, or int16 codes with |lq| < 128) the sum is exact in FP32 and
-// the result equals the FP64 form bit for bit.
+// that is <= 24 (int8 codes, or int16 codes with |lq| < 128) every coordinate is an exact
+// FP32 number on one grid, and so are the differences of coordinates of neighbouring cells,
+// in any order of the sums.
 template <bool FAST>
-__device__ __forceinline__ float pp_xq(const Geo& G, int lq, int code, float xres_f) {
-  if (FAST) {
-    const float f = __fmul_rn(__fadd_rn((float)((uint32_t)code & G.zmask), 0.5f), xres_f);
-    return __fmul_rn(__fadd_rn((float)lq, f), (float)G.rcs);
-  }
+__device__ __forceinline__ float pp_xq(const Geo& G, int lq, int code) {
+  static_assert(!FAST, "the FAST form folds the decode into the difference");
   return __fmul_rn((float)((double)lq + zfrac(code, G)), (float)G.rcs);
 }
 
-template <bool FAST>
-__global__ void k_pp(Geo G, int64_t np, const void* __restrict__ xp, const int32_t* __restrict__ pcell,
-                     const int64_t* __restrict__ cstart, const int32_t* __restrict__ ires, float* __restrict__ vp,
-                     const StepDev* __restrict__ sd, float* f2max, float* vmax,
-                     unsigned long long* npairs, unsigned long long* ncand, const unsigned* __restrict__ abort) {
-  const int64_t ip0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const float mass_scale = sd->pp_mass, v_scale = sd->pp_vscale;
-  // abort: the class lists of a captured step were too short; PM3 is finished for the
-  // unlisted subtiles afterwards and PP must follow it, so PP leaves vp alone here
-  const bool live = ip0 < np && !(abort && *abort) && owned_cell(G, pcell[ip0]);
-  const int64_t ip = live ? ip0 : np - 1;
-  int g[3];
-  cell_coords(G, pcell[ip], g[0], g[1], g[2]);
-  int t[3], u[3], l[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    t[d] = g[d] / G.nt;
-    l[d] = g[d] - t[d] * G.nt;
-    u[d] = l[d] / G.ntt;
-  }
-  const int iapm = ires[subtile_id(G, t, u)];
-  const float xres_f = (float)G.x_res;  // a power of two
-  const float range = __fdiv_rn(3.5f, (float)rsf_of(iapm));  // apm3(iapm)
-  const float range2 = __fmul_rn(range, range);
-  float xf[3], fin[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const double fr = zfrac(load_code(xp, G.izipx, 3 * ip + d), G);
-    xf[d] = __fmul_rn((float)((double)l[d] + fr), (float)G.rcs);  // xvec*ratio_cs (kick.f90:424)
-    fin[d] = __fmul_rn((float)fr, (float)G.rcs);                  // offset inside the coarse cell, fine units
-  }
-  int lo[3], hi[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = (fin[d] < range) ? -1 : 0;
-    hi[d] = ((float)G.rcs - fin[d] < range) ? 1 : 0;
-  }
-  float acc[3] = {0.f, 0.f, 0.f};
-  unsigned long long cnt = 0, cand = 0;
-  if (live)
-  for (int dz = lo[2]; dz <= hi[2]; ++dz)
-    for (int dy = lo[1]; dy <= hi[1]; ++dy)
-      for (int dx = lo[0]; dx <= hi[0]; ++dx) {
-        const int64_t c = nbr_cell(G, pcell[ip], l, g, dx, dy, dz);
-        const int64_t s = cstart[c], e = cstart[c + 1];
-        cand += (unsigned long long)(e - s);
-        const int lq[3] = {l[0] + dx, l[1] + dy, l[2] + dz};
-        for (int64_t q = s; q < e; ++q) {
-          float rv[3];
-#pragma unroll
-          for (int d = 0; d < 3; ++d) rv[d] = __fsub_rn(pp_xq<FAST>(G, lq[d], load_code(xp, G.izipx, 3 * q + d), xres_f), xf[d]);
-          const float r2 = sumsq3(rv[0], rv[1], rv[2]);
-          if (r2 > 0.f && r2 < range2) {
-            const float rm = __fsqrt_rn(r2);
-            const float sc = F_ra(rm, G.app) - F_ra(rm, range);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) acc[d] += __fdiv_rn(rv[d], rm) * sc;
-            ++cnt;
-          }
-        }
-      }
-  float f1[3], av[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-  for (int d = 0; d < 3; ++d) f1[d] = __fmul_rn(acc[d], mass_scale);
-  const float f2 = live ? sumsq3(f1[0], f1[1], f1[2]) : 0.f;
-  if (live) {
+// One particle's PP state: its tile-local position xf (fine cells), the candidate cell
+// range per dimension, its range and the accumulated force.
+struct PPi {
+  float xf[3];
+  int l[3], lo[3], hi[3];
+  float range, range2;
+  float k_range, c_range, p_range;  // 2/range, (1/35)/range^2, 3 range^2: F_s2 of the range
+  float k_app, c_app, p_app;        // the same of the softening app (k_app infinite: none)
+  float acc[3];
+  unsigned pairs, cand;  // of this particle (item): well below 2^32
+
+  __device__ __forceinline__ void init(const Geo& G, const int g[3], const float4 fin, int iapm) {
+    const float fi[3] = {fin.x, fin.y, fin.z};
+    range = __fdiv_rn(3.5f, (float)rsf_of(iapm));  // apm3(iapm)
+    range2 = __fmul_rn(range, range);
+    k_range = __fdiv_rn(2.f, range);
+    c_range = __fdiv_rn(__fdiv_rn(1.f, 35.f), range2);
+    p_range = 3.f * range2;
+    k_app = G.app > 0.f ? __fdiv_rn(2.f, G.app) : __int_as_float(0x7f800000);
+    c_app = G.app > 0.f ? __fdiv_rn(__fdiv_rn(1.f, 35.f), __fmul_rn(G.app, G.app)) : 0.f;
+    p_app = 3.f * G.app * G.app;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
+      l[d] = g[d] % G.nt;
+      xf[d] = __fadd_rn((float)(l[d] * G.rcs), fi[d]);
+      lo[d] = (fi[d] < range) ? -1 : 0;
+      hi[d] = ((float)G.rcs - fi[d] < range) ? 1 : 0;
+      acc[d] = 0.f;
+    }
+    pairs = cand = 0;
+  }
+
+  __device__ __forceinline__ bool needs(int dx, int dy, int dz) const {
+    return dx >= lo[0] && dx <= hi[0] && dy >= lo[1] && dy <= hi[1] && dz >= lo[2] && dz <= hi[2];
+  }
+
+  // The force of one pair in range (separation rv, r2 = |rv|^2) added to acc, in the order
+  // the callers call it (candidate order).  1/r is the hardware's approximate reciprocal
+  // square root and one Newton step (y + y (1/2 - r2 y^2 / 2)), good to about one unit in the
+  // last place; the force law and the projection multiply by it.  With IEEE square root and
+  // divisions (up to eight a pair) the law took three times the instructions (with the packed
+  // separations, the heavy-cell PP of 128^3 clustered particles: 24.8 -> 13.4 ms); the force's
+  // error against 64 bits is the same.
+  __device__ __forceinline__ void accum(float rv0, float rv1, float rv2, float r2) {
+    const float y = rsqrtf(r2);
+    const float inv = __fmaf_rn(y, __fmaf_rn(__fmul_rn(__fmul_rn(-0.5f, r2), y), y, 0.5f), y);
+    const float inv2 = __fmul_rn(inv, inv), r = __fmul_rn(r2, inv);
+    float sc = inv2;
+    const float ea = __fmul_rn(r, k_app);
+    if (ea <= 2.f) sc = F_s2(ea, c_app, __fmul_rn(p_app, inv2));
+    sc = __fsub_rn(sc, F_s2(__fmul_rn(r, k_range), c_range, __fmul_rn(p_range, inv2)));
+    sc = __fmul_rn(sc, inv);
+    acc[0] = __fmaf_rn(rv0, sc, acc[0]);
+    acc[1] = __fmaf_rn(rv1, sc, acc[1]);
+    acc[2] = __fmaf_rn(rv2, sc, acc[2]);
+  }
+};
+
+// Two FP32 operations in one instruction (sm_100's packed form), lane by lane the same as
+// the scalar ones.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return reinterpret_cast<const float2&>(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return reinterpret_cast<const float2&>(r);
+}
+
+// The plain form: one thread per particle over the coarse cells its range reaches, reading
+// the candidates' codes.  Candidates go four at a time as independent chains; pairs in range
+// are kept in the thread's own shared-memory column and added with PPi::accum in candidate
+// order when it may run full and at the end, so that the lanes of a warp evaluate their
+// pairs together (128^3 particles at 8 a cell: 0.76 -> 0.42 ms; at 64 a cell with cells of up
+// to 4e3: 14.5 -> 12.3 ms, bound by the lanes' different neighbour cells).
+constexpr int PP_T = 128, PP_H = 8, PP_U = 4;
+template <bool FAST, typename CODE>
+__global__ void __launch_bounds__(PP_T) k_pp(Geo G, int64_t np, const CODE* __restrict__ xp,
+                                             const int32_t* __restrict__ pcell, const int64_t* __restrict__ cstart,
+                                             const int32_t* __restrict__ ires, float* __restrict__ vp,
+                                             const StepDev* __restrict__ sd, float* f2max, float* vmax,
+                                             unsigned long long* npairs, unsigned long long* ncand,
+                                             const unsigned* __restrict__ abort) {
+  __shared__ float4 hb[PP_H][PP_T];
+  const int64_t ip = (int64_t)blockIdx.x * PP_T + threadIdx.x;
+  // abort: the class lists of a captured step were too short; PM3 is finished for the
+  // unlisted subtiles afterwards and PP must follow it, so PP leaves vp alone here
+  bool live = ip < np && !(abort && *abort);
+  int c = 0;
+  if (live) {
+    c = pcell[ip];
+    live = owned_cell(G, c);
+  }
+  float f2 = 0.f, av[3] = {0.f, 0.f, 0.f};
+  PPi P;
+  P.pairs = P.cand = 0;
+  if (live) {
+    int g[3];
+    cell_coords(G, c, g[0], g[1], g[2]);
+    int t[3], u[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      t[d] = g[d] / G.nt;
+      u[d] = (g[d] - t[d] * G.nt) / G.ntt;
+    }
+    float fin[3], xf[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double fr = zfrac((int)xp[3 * ip + d], G);
+      fin[d] = __fmul_rn((float)fr, (float)G.rcs);  // offset inside the coarse cell, fine units
+      xf[d] = __fmul_rn((float)((double)(g[d] - t[d] * G.nt) + fr), (float)G.rcs);  // xvec*ratio_cs (kick.f90:424)
+    }
+    P.init(G, g, make_float4(fin[0], fin[1], fin[2], 0.f), ires[subtile_id(G, t, u)]);
+    if (!FAST) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) P.xf[d] = xf[d];
+    }
+    const float step = (float)(G.x_res * (double)G.rcs);  // fine cells per code unit, a power of two
+    int nh = 0;
+    for (int dz = P.lo[2]; dz <= P.hi[2]; ++dz)
+      for (int dy = P.lo[1]; dy <= P.hi[1]; ++dy)
+        for (int dx = P.lo[0]; dx <= P.hi[0]; ++dx) {
+          const int64_t n = nbr_cell(G, c, P.l, g, dx, dy, dz);
+          const int64_t s = cstart[n], e = cstart[n + 1];
+          P.cand += (unsigned)(e - s);
+          const int lq[3] = {P.l[0] + dx, P.l[1] + dy, P.l[2] + dz};
+          float base[3];  // cell corner plus half a code unit, less xf: exact when FAST
+#pragma unroll
+          for (int d = 0; d < 3; ++d) base[d] = (float)(lq[d] * G.rcs) - P.xf[d] + 0.5f * step;
+          for (int64_t q0 = s; q0 < e; q0 += PP_U) {
+            float rv[PP_U][3], r2[PP_U];
+            bool hit[PP_U];
+#pragma unroll
+            for (int k = 0; k < PP_U; ++k) {
+              const bool valid = q0 + k < e;
+              const CODE* cp = xp + 3 * (valid ? q0 + k : q0);
+#pragma unroll
+              for (int d = 0; d < 3; ++d)
+                rv[k][d] = FAST ? fmaf((float)cp[d], step, base[d]) : __fsub_rn(pp_xq<false>(G, lq[d], (int)cp[d]), P.xf[d]);
+              r2[k] = sumsq3(rv[k][0], rv[k][1], rv[k][2]);
+              hit[k] = valid && r2[k] > 0.f && r2[k] < P.range2;
+            }
+#pragma unroll
+            for (int k = 0; k < PP_U; ++k)
+              if (hit[k]) {
+                if (nh == PP_H) {
+#pragma unroll 1
+                  for (int h = 0; h < PP_H; ++h) {
+                    const float4 r = hb[h][threadIdx.x];
+                    P.accum(r.x, r.y, r.z, r.w);
+                  }
+                  nh = 0;
+                }
+                hb[nh][threadIdx.x] = make_float4(rv[k][0], rv[k][1], rv[k][2], r2[k]);
+                ++nh;
+                ++P.pairs;
+              }
+          }
+        }
+#pragma unroll 1
+    for (int h = 0; h < nh; ++h) {
+      const float4 r = hb[h][threadIdx.x];
+      P.accum(r.x, r.y, r.z, r.w);
+    }
+    float f1[3];
+    const float mass_scale = sd->pp_mass, v_scale = sd->pp_vscale;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      f1[d] = __fmul_rn(P.acc[d], mass_scale);
       const float v = __fadd_rn(vp[3 * ip + d], __fmul_rn(f1[d], v_scale));
       vp[3 * ip + d] = v;
       av[d] = fabsf(v);
     }
+    f2 = sumsq3(f1[0], f1[1], f1[2]);
   }
   block_max_to(f2, f2max);
   block_vmax(av, vmax);
-  unsigned long long c = live ? cnt : 0ull, cd = live ? cand : 0ull;
+  unsigned long long a = P.pairs, b = P.cand;  // warp sums in 64 bits
   for (int o = 16; o > 0; o >>= 1) {
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-    cd += __shfl_xor_sync(0xffffffffu, cd, o);
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
   }
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(npairs, c);
-  if ((threadIdx.x & 31) == 0 && cd) atomicAdd(ncand, cd);
+  if ((threadIdx.x & 31) == 0 && a) atomicAdd(npairs, a);
+  if ((threadIdx.x & 31) == 0 && b) atomicAdd(ncand, b);
 }
 
 // =================================================================================

@@ -34,78 +34,6 @@ __global__ void k_ppq_prep(Geo G, int64_t np, const void* __restrict__ xp, float
   pfin[ip] = make_float4(f[0], f[1], f[2], 0.f);
 }
 
-// One particle's PP state: its tile-local position xf (fine cells), the candidate cell
-// range per dimension, its range and the accumulated force.  The candidate coordinate is
-// (lq*ratio_cs) + offset with lq = l + d: exact in FP32 when lq + offset fits 24 bits (the
-// FAST case of k_pp), so rv equals k_pp's FAST arithmetic bit for bit.
-struct PPi {
-  float xf[3];
-  int l[3], lo[3], hi[3];
-  float range, range2, coef_range, coef_app;  // range and F_ra_coef of range and app
-  float acc[3];
-  unsigned pairs, cand;  // of this particle (item): well below 2^32
-
-  __device__ __forceinline__ void init(const Geo& G, const int g[3], const float4 fin, int iapm) {
-    const float fi[3] = {fin.x, fin.y, fin.z};
-    range = __fdiv_rn(3.5f, (float)rsf_of(iapm));  // apm3(iapm)
-    range2 = __fmul_rn(range, range);
-    coef_range = F_ra_coef(range);
-    coef_app = F_ra_coef(G.app);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      l[d] = g[d] % G.nt;
-      xf[d] = __fadd_rn((float)(l[d] * G.rcs), fi[d]);
-      lo[d] = (fi[d] < range) ? -1 : 0;
-      hi[d] = ((float)G.rcs - fi[d] < range) ? 1 : 0;
-      acc[d] = 0.f;
-    }
-    pairs = cand = 0;
-  }
-
-  __device__ __forceinline__ bool needs(int dx, int dy, int dz) const {
-    return dx >= lo[0] && dx <= hi[0] && dy >= lo[1] && dy <= hi[1] && dz >= lo[2] && dz <= hi[2];
-  }
-
-  // The force of one pair in range (separation rv, r2 = |rv|^2) added to acc.  Callers
-  // that defer their pairs call it in candidate order, so the sums are k_pp's.
-  __device__ __forceinline__ void accum(float rv0, float rv1, float rv2, float r2, float app) {
-    const float rm = __fsqrt_rn(r2);
-    const float sc = __fsub_rn(F_ra_c(rm, app, coef_app), F_ra_c(rm, range, coef_range));
-    acc[0] = __fadd_rn(acc[0], __fmul_rn(__fdiv_rn(rv0, rm), sc));
-    acc[1] = __fadd_rn(acc[1], __fmul_rn(__fdiv_rn(rv1, rm), sc));
-    acc[2] = __fadd_rn(acc[2], __fmul_rn(__fdiv_rn(rv2, rm), sc));
-  }
-
-  // One candidate at in-cell offset p of the neighbour cell whose tile-local coarse
-  // coordinates are (bx, by, bz) (= l + d), already multiplied by ratio_cs.
-  __device__ __forceinline__ void pair(float bx, float by, float bz, const float4 p, float app) {
-    const float rv0 = __fsub_rn(__fadd_rn(bx, p.x), xf[0]);
-    const float rv1 = __fsub_rn(__fadd_rn(by, p.y), xf[1]);
-    const float rv2 = __fsub_rn(__fadd_rn(bz, p.z), xf[2]);
-    const float r2 = sumsq3(rv0, rv1, rv2);
-    if (r2 > 0.f && r2 < range2) {
-      accum(rv0, rv1, rv2, r2, app);
-      ++pairs;
-    }
-  }
-
-  // The candidates of every cell this particle's range reaches, in order (the sums of
-  // k_pp), reading the decoded offsets; counts candidates.  c: the particle's storage cell.
-  __device__ __forceinline__ void all_cells(const Geo& G, int64_t c, const int g[3], const int64_t* __restrict__ cstart,
-                                            const float4* __restrict__ pfin) {
-    for (int dz = lo[2]; dz <= hi[2]; ++dz)
-      for (int dy = lo[1]; dy <= hi[1]; ++dy)
-        for (int dx = lo[0]; dx <= hi[0]; ++dx) {
-          const int64_t n = nbr_cell(G, c, l, g, dx, dy, dz);
-          const int64_t s = cstart[n], e = cstart[n + 1];
-          cand += (unsigned)(e - s);
-          const float bx = (float)((l[0] + dx) * G.rcs), by = (float)((l[1] + dy) * G.rcs),
-                      bz = (float)((l[2] + dz) * G.rcs);
-          for (int64_t q = s; q < e; ++q) pair(bx, by, bz, pfin[q], G.app);
-        }
-  }
-};
-
 // The kick of one particle from its PP force (kick.f90:300-306); returns |F|^2 and |v|.
 __device__ __forceinline__ float ppq_apply(const PPi& P, int64_t ip, const float* vin, float* vout, float mass_scale,
                                            float v_scale, float av[3]) {
@@ -169,8 +97,9 @@ __global__ void __launch_bounds__(PPL_T) k_ppq_light(Geo G, int64_t np, const in
           const int64_t n = nbr_cell(G, c, P.l, g, dx, dy, dz);
           const int64_t s = cstart[n], e = cstart[n + 1];
           P.cand += (unsigned)(e - s);
-          const float bx = (float)((P.l[0] + dx) * G.rcs), by = (float)((P.l[1] + dy) * G.rcs),
-                      bz = (float)((P.l[2] + dz) * G.rcs);
+          // the cell's corner less xf, exact: a separation is one sum with the offset
+          const float2 txy = make_float2((float)((P.l[0] + dx) * G.rcs) - P.xf[0], (float)((P.l[1] + dy) * G.rcs) - P.xf[1]);
+          const float tz = (float)((P.l[2] + dz) * G.rcs) - P.xf[2];
           for (int64_t q0 = s; q0 < e; q0 += PPL_U) {
             // PPL_U candidates as independent chains (loads in flight together, the tail
             // predicated off), their pairs then recorded in candidate order
@@ -180,10 +109,11 @@ __global__ void __launch_bounds__(PPL_T) k_ppq_light(Geo G, int64_t np, const in
             for (int u = 0; u < PPL_U; ++u) {
               const bool valid = q0 + u < e;
               const float4 p = pfin[valid ? q0 + u : q0];
-              rv[u][0] = __fsub_rn(__fadd_rn(bx, p.x), P.xf[0]);
-              rv[u][1] = __fsub_rn(__fadd_rn(by, p.y), P.xf[1]);
-              rv[u][2] = __fsub_rn(__fadd_rn(bz, p.z), P.xf[2]);
-              r2[u] = sumsq3(rv[u][0], rv[u][1], rv[u][2]);
+              const float2 rxy = add2(txy, make_float2(p.x, p.y)), sq = mul2(rxy, rxy);
+              rv[u][0] = rxy.x;
+              rv[u][1] = rxy.y;
+              rv[u][2] = __fadd_rn(tz, p.z);
+              r2[u] = __fadd_rn(__fadd_rn(sq.x, sq.y), __fmul_rn(rv[u][2], rv[u][2]));
               hit[u] = valid && r2[u] > 0.f && r2[u] < P.range2;
             }
 #pragma unroll
@@ -193,7 +123,7 @@ __global__ void __launch_bounds__(PPL_T) k_ppq_light(Geo G, int64_t np, const in
 #pragma unroll 1
                   for (int h = 0; h < PPL_H; ++h) {
                     const float4 r = hb[h][threadIdx.x];
-                    P.accum(r.x, r.y, r.z, r.w, G.app);
+                    P.accum(r.x, r.y, r.z, r.w);
                   }
                   nh = 0;
                 }
@@ -206,7 +136,7 @@ __global__ void __launch_bounds__(PPL_T) k_ppq_light(Geo G, int64_t np, const in
 #pragma unroll 1
     for (int h = 0; h < nh; ++h) {
       const float4 r = hb[h][threadIdx.x];
-      P.accum(r.x, r.y, r.z, r.w, G.app);
+      P.accum(r.x, r.y, r.z, r.w);
     }
     f2 = ppq_apply(P, ip, vin, vout, sd->pp_mass, sd->pp_vscale, av);
   }
@@ -353,8 +283,11 @@ __global__ void __launch_bounds__(256) k_ppq_sort_codes(Geo G, const int32_t* __
 constexpr int PPH_H = 8;   // deferred pairs per thread
 constexpr int PPH_U = 4;   // candidates between checks of the deferred count
 
+// Candidates staged per chunk, up to whole groups (16-byte reads of x, y and z).
+__host__ __device__ inline int ppq_chunk_pitch(int J) { return (J + PPH_U - 1) / PPH_U * PPH_U; }
+
 __host__ __device__ inline size_t ppq_heavy_smem(int B, int J) {
-  return (size_t)J * sizeof(float4) + (size_t)PPH_H * B * sizeof(float4);
+  return (size_t)PPH_H * B * sizeof(float4) + (size_t)3 * ppq_chunk_pitch(J) * sizeof(float);
 }
 
 __global__ void k_ppq_heavy(Geo G, const int32_t* __restrict__ hlist, const int* __restrict__ hpre, int* q,
@@ -362,10 +295,13 @@ __global__ void k_ppq_heavy(Geo G, const int32_t* __restrict__ hlist, const int*
                             const float4* __restrict__ pfin, const int32_t* __restrict__ hperm, const float* vin,
                             float* vout, const StepDev* __restrict__ sd, int J, float* f2max, float* vmax,
                             unsigned long long* npairs, unsigned long long* ncand, const unsigned* __restrict__ abort) {
-  extern __shared__ float4 sj[];  // J candidates, then the deferred pairs [PPH_H][B]
+  extern __shared__ float4 sj[];  // the deferred pairs [PPH_H][B], then x, y, z of JP candidates
   __shared__ int s_item;
-  const int B = blockDim.x;
-  float4* const hb = sj + J;
+  const int B = blockDim.x, JP = ppq_chunk_pitch(J);
+  float4* const hb = sj;
+  float* const sx = reinterpret_cast<float*>(sj + PPH_H * B);
+  float* const sy = sx + JP;
+  float* const sz = sy + JP;
   const bool aborted = abort && *abort;
   const int nh = q[64], nitems = q[65];
   const float mass_scale = sd->pp_mass, v_scale = sd->pp_vscale;
@@ -398,8 +334,9 @@ __global__ void k_ppq_heavy(Geo G, const int32_t* __restrict__ hlist, const int*
 #pragma unroll 1
       for (int h = 0; h < nh; ++h) {
         const float4 r = hb[h * B + threadIdx.x];
-        P.accum(r.x, r.y, r.z, r.w, G.app);
+        P.accum(r.x, r.y, r.z, r.w);
       }
+      P.pairs += nh;
       nh = 0;
     };
     for (int dz = -1; dz <= 1; ++dz)
@@ -410,37 +347,49 @@ __global__ void k_ppq_heavy(Geo G, const int32_t* __restrict__ hlist, const int*
           const int64_t n = nbr_cell(G, c, P.l, g, dx, dy, dz);
           const int64_t s = cstart[n], e = cstart[n + 1];
           if (need) P.cand += (unsigned)(e - s);
-          const float bx = (float)((P.l[0] + dx) * G.rcs), by = (float)((P.l[1] + dy) * G.rcs),
-                      bz = (float)((P.l[2] + dz) * G.rcs);
+          // the cell's corner less xf, exact: a separation is one sum with the offset
+          const float tx = (float)((P.l[0] + dx) * G.rcs) - P.xf[0], ty = (float)((P.l[1] + dy) * G.rcs) - P.xf[1],
+                      tz = (float)((P.l[2] + dz) * G.rcs) - P.xf[2];
+          const float2 tx2 = make_float2(tx, tx), ty2 = make_float2(ty, ty), tz2 = make_float2(tz, tz);
           for (int64_t j0 = s; j0 < e; j0 += J) {
             const int cnt = (int)((e - j0) < (int64_t)J ? (e - j0) : (int64_t)J);
             __syncthreads();
-            for (int k = threadIdx.x; k < cnt; k += B) sj[k] = pfin[j0 + k];
+            for (int k = threadIdx.x; k < cnt; k += B) {
+              const float4 p = pfin[j0 + k];
+              sx[k] = p.x;
+              sy[k] = p.y;
+              sz[k] = p.z;
+            }
+            if (threadIdx.x < PPH_U)  // the group's tail: a candidate out of every range
+              for (int k = cnt + threadIdx.x; k < ((cnt + PPH_U - 1) & ~(PPH_U - 1)); k += PPH_U)
+                sx[k] = sy[k] = sz[k] = 1e9f;
             __syncthreads();
             if (__any_sync(0xffffffffu, need))  // warp-uniform
             for (int k0 = 0; k0 < cnt; k0 += PPH_U) {
               if (need) {
-                // PPH_U candidates as independent chains (the tail predicated off), their
-                // pairs then recorded in candidate order
-                float rv[PPH_U][3], r2[PPH_U];
-                bool hit[PPH_U];
+                // PPH_U candidates, two to an instruction, their pairs then recorded in
+                // candidate order
+                const float4 px = *reinterpret_cast<const float4*>(sx + k0);
+                const float4 py = *reinterpret_cast<const float4*>(sy + k0);
+                const float4 pz = *reinterpret_cast<const float4*>(sz + k0);
+                const float2 rx[2] = {add2(tx2, make_float2(px.x, px.y)), add2(tx2, make_float2(px.z, px.w))};
+                const float2 ry[2] = {add2(ty2, make_float2(py.x, py.y)), add2(ty2, make_float2(py.z, py.w))};
+                const float2 rz[2] = {add2(tz2, make_float2(pz.x, pz.y)), add2(tz2, make_float2(pz.z, pz.w))};
 #pragma unroll
-                for (int q = 0; q < PPH_U; ++q) {
-                  const bool valid = k0 + q < cnt;
-                  const float4 p = sj[valid ? k0 + q : k0];
-                  rv[q][0] = __fsub_rn(__fadd_rn(bx, p.x), P.xf[0]);
-                  rv[q][1] = __fsub_rn(__fadd_rn(by, p.y), P.xf[1]);
-                  rv[q][2] = __fsub_rn(__fadd_rn(bz, p.z), P.xf[2]);
-                  r2[q] = sumsq3(rv[q][0], rv[q][1], rv[q][2]);
-                  hit[q] = valid && r2[q] > 0.f && r2[q] < P.range2;
-                }
-#pragma unroll
-                for (int q = 0; q < PPH_U; ++q)
-                  if (hit[q]) {
-                    hb[nh * B + threadIdx.x] = make_float4(rv[q][0], rv[q][1], rv[q][2], r2[q]);
+                for (int q = 0; q < 2; ++q) {
+                  // sums of the squares one by one: two packed operations in a row may be
+                  // contracted, and the range test has to see sumsq3's rounding
+                  const float2 xx = mul2(rx[q], rx[q]), yy = mul2(ry[q], ry[q]), zz = mul2(rz[q], rz[q]);
+                  const float2 r2 = make_float2(__fadd_rn(__fadd_rn(xx.x, yy.x), zz.x), __fadd_rn(__fadd_rn(xx.y, yy.y), zz.y));
+                  if (r2.x > 0.f && r2.x < P.range2) {
+                    hb[nh * B + threadIdx.x] = make_float4(rx[q].x, ry[q].x, rz[q].x, r2.x);
                     ++nh;
-                    ++P.pairs;
                   }
+                  if (r2.y > 0.f && r2.y < P.range2) {
+                    hb[nh * B + threadIdx.x] = make_float4(rx[q].y, ry[q].y, rz[q].y, r2.y);
+                    ++nh;
+                  }
+                }
               }
               if (__any_sync(0xffffffffu, nh > PPH_H - PPH_U)) flush();
             }

@@ -135,6 +135,31 @@ __device__ __forceinline__ unsigned long long fixed40(float w) {
   return (unsigned long long)__float2ll_rn(__fmul_rn(w, 1099511627776.f));
 }
 
+// Two FP32 operations in one instruction (sm_100's packed form), lane by lane the same as
+// the scalar ones, except that a product and a sum that follow each other may be contracted.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return reinterpret_cast<const float2&>(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return reinterpret_cast<const float2&>(r);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r)
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+        "l"(reinterpret_cast<const unsigned long long&>(c)));
+  return reinterpret_cast<const float2&>(r);
+}
+
 // Non-negative float max through integer atomics.
 __device__ __forceinline__ void atomic_max_pos(float* addr, float v) {
   atomicMax(reinterpret_cast<int*>(addr), __float_as_int(v));

@@ -396,7 +396,7 @@ Geo make_geo(const cube_params& p) {
 }
 
 // In-place mesh layouts (fft2.cuh): boxes of side n are n planes of `psb` bytes.
-//  row-pitched: rows of RP = max(n*rb, (n/2+1)*8) bytes, psb = n*RP;
+//  row-pitched: rows of RP = max(n*rb, (n/2+1)*8) bytes, rounded up to 16, psb = n*RP;
 //  plane-compact (sizes that run the fused plane FFT): rows of n reals / n/2+1 complex /
 //    n floats from the start of the plane, psb = max(n*n*rb, n*(n/2+1)*8).
 // rb = 4, or 8 for the int64 fixed-point deposit.
@@ -419,7 +419,7 @@ Pitch pitch_of(const cube_ctx* c, int n, bool fixed) {
     p.pf = n;
     p.rp = n * rb;
   } else {
-    p.rp = std::max<int64_t>((int64_t)n * rb, nh * 8);
+    p.rp = (std::max<int64_t>((int64_t)n * rb, nh * 8) + 15) & ~(int64_t)15;
     p.psb = n * p.rp;
     p.pr = (int)(p.rp / rb);
     p.pc = (int)(p.rp / 8);
@@ -1452,7 +1452,8 @@ static int enqueue_kick_a(cube_ctx* c) {
       if (c->cap_level == 2 && c->cap_box >= t0 && c->cap_box < t0 + nb)
         maybe_capture(c, 2, c->cap_box, 1, (char*)m.real + (c->cap_box - t0) * boxb, n, false, (int64_t)m.pt.pf * 4,
                       m.pt.psb);
-      LAUNCH(c, K_F2_PM2, 1, k_f2max_box2<<<f2max_box2_grid(G.ngp, nb), 256, 0, c->s>>>(phi, n, G.ngp, 1 - G.ngb, nb, f2 + 1, m.pt.pf, m.pt.plf, nullptr));
+      auto kf2 = f2max_box3_fits(n, G.ngp, 1 - G.ngb, m.pt.pf, m.pt.plf, phi) ? k_f2max_box3 : k_f2max_box2;
+      LAUNCH(c, K_F2_PM2, 1, kf2<<<f2max_box2_grid(G.ngp, nb), 256, 0, c->s>>>(phi, n, G.ngp, 1 - G.ngb, nb, f2 + 1, m.pt.pf, m.pt.plf, nullptr));
       LAUNCH(c, K_INT_PM2, 1, k_interp_pm2<<<nblk(np), 256, 0, c->s>>>(G, np, c->xp, c->pcell, phi, t0, nb, c->vp, c->sd, vm + 0, c->err, m.pt.pf, m.pt.plf));
     }
   }
@@ -1597,7 +1598,8 @@ static int enqueue_pm3(cube_ctx* c, const PM3Plan& pl, bool host_ires) {
       if (cap_here)
         maybe_capture(c, 3, c->cap_box, 1, (char*)m.real + cap_slot * boxb, n, false, (int64_t)m.pt.pf * 4, m.pt.psb);
       const int nf = G.nfp[cl];
-      LAUNCH(c, K_F2_PM3, 1, k_f2max_box2<<<f2max_box2_grid(nf, nb), 256, 0, c->s>>>(phi, n, nf, 1 - G.nfb[cl], nb, f2 + 2, m.pt.pf, m.pt.plf, subs));
+      auto kf3 = f2max_box3_fits(n, nf, 1 - G.nfb[cl], m.pt.pf, m.pt.plf, phi) ? k_f2max_box3 : k_f2max_box2;
+      LAUNCH(c, K_F2_PM3, 1, kf3<<<f2max_box2_grid(nf, nb), 256, 0, c->s>>>(phi, n, nf, 1 - G.nfb[cl], nb, f2 + 2, m.pt.pf, m.pt.plf, subs));
       unsigned long long* ms3 = c->msum + 2 * MASS_SLOTS * MASS_STRIDE;
       if (fixed)
         LAUNCH(c, K_INT_PM3, 1, k_interp_pm3<true><<<nblk(np), 256, 0, c->s>>>(G, np, c->xp, c->pcell, phi, slots, cl, c->vp,

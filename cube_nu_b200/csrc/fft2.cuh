@@ -179,7 +179,7 @@ __device__ __forceinline__ void seq_transform_g(float2* base, int se, int t, con
 }
 
 // Mesh layouts (both in place, potential written over the input):
-//  row-pitched (five-pass sizes): row pitch RP bytes = max(N*rb, (N/2+1)*8), so a real
+//  row-pitched (five-pass sizes): row pitch RP bytes = max(N*rb, (N/2+1)*8) up to 16, so a real
 //    row and its half-spectrum row share bytes (FFTW's in-place r2c layout); plane = N rows;
 //  plane-compact (fused sizes): real rows of N, half-spectrum rows of N/2+1 and phi rows of
 //    N packed from the start of each plane; plane pitch max(N*N*rb, N*(N/2+1)*8) bytes.

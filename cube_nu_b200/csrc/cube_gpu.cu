@@ -397,8 +397,8 @@ Geo make_geo(const cube_params& p) {
 
 // In-place mesh layouts (fft2.cuh): boxes of side n are n planes of `psb` bytes.
 //  row-pitched: rows of RP = max(n*rb, (n/2+1)*8) bytes, rounded up to 16, psb = n*RP;
-//  plane-compact (sizes that run the fused plane FFT): rows of n reals / n/2+1 complex /
-//    n floats from the start of the plane, psb = max(n*n*rb, n*(n/2+1)*8).
+//  plane-compact (sizes that run the fused plane FFT): rows of n reals / n/2+1 complex up to
+//    even / n floats from the start of the plane, psb the larger of the two.
 // rb = 4, or 8 for the int64 fixed-point deposit.
 struct Pitch {
   int64_t rp;    // bytes per real row (capture copies)
@@ -413,9 +413,9 @@ Pitch pitch_of(const cube_ctx* c, int n, bool fixed) {
   const int64_t rb = fixed ? 8 : 4, nh = n / 2 + 1;
   Pitch p;
   if (fused_layout(c, n)) {
-    p.psb = std::max<int64_t>((int64_t)n * n * rb, (int64_t)n * nh * 8);
+    p.pc = (int)(nh + 1) / 2 * 2;
+    p.psb = std::max<int64_t>((int64_t)n * n * rb, (int64_t)n * p.pc * 8);
     p.pr = n;
-    p.pc = (int)nh;
     p.pf = n;
     p.rp = n * rb;
   } else {
@@ -520,10 +520,11 @@ void fft2_run(cube_ctx* c, int64_t nbox, const void* real_in, bool fixed, float 
         LAUNCH(c, kx, 1, f2::k_fxy3_r2c<N, R1, R2, float><<<planes, f2::PlaneShape<N, R1, R2>::THREADS, smf, c->s>>>(
                              (const float*)real_in, ck, tw, scale, pt.pr, pt.pc, pt.plr, pt.plc));
       }
-      // plane sizes: the block-per-line column pass hides latency with more warps
-      const size_t smg = smc + (size_t)W * N * sizeof(float);  // + prefetched Green values
-      smem_optin(f2::k_fcol3<N, R1, R2, 2, 2>, smg);
-      LAUNCH(c, kz, 1, f2::k_fcol3<N, R1, R2, 2, 2><<<gc, W * T, smg, c->s>>>(ck, green, tw, W, pt.pc, pt.plc));
+      using Z = f2::ZLoop<N, R1, R2>;
+      const int lines = N * Z::NCG, ns = f2::fz_loop_split(lines, c->nsm * Z::MINB, nbox);
+      auto zl = f2::k_fz_loop<N, R1, R2>;
+      smem_optin(zl, Z::SMEM);
+      LAUNCH(c, kz, 1, zl<<<(unsigned)(lines * ns), Z::THREADS, Z::SMEM, c->s>>>(ck, green, tw, pt.pc, pt.plc, nbox, ns));
       smem_optin(f2::k_fyx3_c2r<N, R1, R2>, smi);
       LAUNCH(c, kc, 1, f2::k_fyx3_c2r<N, R1, R2><<<planes, f2::PlaneShape<N, R1, R2>::THREADS, smi, c->s>>>(
                            ck, phi_out, tw, inv, pt.pc, pt.pf, pt.plc, pt.plf));
@@ -545,9 +546,9 @@ void fft2_run(cube_ctx* c, int64_t nbox, const void* real_in, bool fixed, float 
   smem_optin(f2::k_fcol3<N, R1, R2, 1, 0>, smc);
   smem_optin(f2::k_fcol3<N, R1, R2, 1, 1>, smc);
   smem_optin(f2::k_fx_c2r<N, R1, R2>, smx);
-  LAUNCH(c, ky, 1, f2::k_fcol3<N, R1, R2, 1, 0><<<gc, W * T, smc, c->s>>>(ck, nullptr, tw, W, pt.pc, pt.plc));
+  LAUNCH(c, ky, 1, f2::k_fcol3<N, R1, R2, 1, 0><<<gc, W * T, smc, c->s>>>(ck, tw, W, pt.pc, pt.plc));
   fz_green<N, R1, R2>(c, nbox, ck, green, tw, pt, kz);
-  LAUNCH(c, ky, 1, f2::k_fcol3<N, R1, R2, 1, 1><<<gc, W * T, smc, c->s>>>(ck, nullptr, tw, W, pt.pc, pt.plc));
+  LAUNCH(c, ky, 1, f2::k_fcol3<N, R1, R2, 1, 1><<<gc, W * T, smc, c->s>>>(ck, tw, W, pt.pc, pt.plc));
   LAUNCH(c, kc, 1, f2::k_fx_c2r<N, R1, R2><<<gx, S * T, smx, c->s>>>(ck, phi_out, nrows, tw, inv, pt.pc, pt.pf));
 }
 
@@ -605,7 +606,7 @@ void fft2_forward(cube_ctx* c, float* real, const Pitch& pt, int cls) {
       smem_optin(f2::k_fxy3_r2c<N, R1, R2, float>, smf);
       LAUNCH(c, cls, 1, f2::k_fxy3_r2c<N, R1, R2, float><<<(unsigned)N, f2::PlaneShape<N, R1, R2>::THREADS, smf, c->s>>>(
                             real, ck, tw, 1.f, pt.pr, pt.pc, pt.plr, pt.plc));
-      LAUNCH(c, cls, 1, f2::k_fcol3<N, R1, R2, 2, 0><<<gc, W * T, smc, c->s>>>(ck, nullptr, tw, W, pt.pc, pt.plc));
+      LAUNCH(c, cls, 1, f2::k_fcol3<N, R1, R2, 2, 0><<<gc, W * T, smc, c->s>>>(ck, tw, W, pt.pc, pt.plc));
       return;
     }
   }
@@ -615,8 +616,8 @@ void fft2_forward(cube_ctx* c, float* real, const Pitch& pt, int cls) {
   smem_optin(f2::k_fx_r2c<N, R1, R2, float>, smx);
   smem_optin(f2::k_fcol3<N, R1, R2, 1, 0>, smc);
   LAUNCH(c, cls, 1, f2::k_fx_r2c<N, R1, R2, float><<<gx, S * T, smx, c->s>>>(real, ck, nrows, tw, 1.f, pt.pr, pt.pc));
-  LAUNCH(c, cls, 1, f2::k_fcol3<N, R1, R2, 1, 0><<<gc, W * T, smc, c->s>>>(ck, nullptr, tw, W, pt.pc, pt.plc));
-  LAUNCH(c, cls, 1, f2::k_fcol3<N, R1, R2, 2, 0><<<gc, W * T, smc, c->s>>>(ck, nullptr, tw, W, pt.pc, pt.plc));
+  LAUNCH(c, cls, 1, f2::k_fcol3<N, R1, R2, 1, 0><<<gc, W * T, smc, c->s>>>(ck, tw, W, pt.pc, pt.plc));
+  LAUNCH(c, cls, 1, f2::k_fcol3<N, R1, R2, 2, 0><<<gc, W * T, smc, c->s>>>(ck, tw, W, pt.pc, pt.plc));
 }
 
 // Forward-only r2c with the generic Stockham passes (any 2^a 3^b size, row-pitched layout):

@@ -13,8 +13,10 @@
 // Passes:
 //   k_fx_r2c   : rows of reals, two rows packed as one complex sequence, unpacked into
 //                two half spectra (r2c)
-//   k_fcol3    : columns (y or z) of the half spectrum, forward / inverse, or forward ->
-//                Green multiply -> inverse (z pass); sequences stay in registers
+//   k_fcol3    : columns (y or z) of the half spectrum, forward / inverse; sequences stay in
+//                registers
+//   k_fz_loop  : z pass, forward -> Green multiply -> inverse, for N <= 144
+//   k_fz_stream: the same for larger N
 //   k_fx_c2r   : two half-spectrum rows packed as one Hermitian-extended sequence,
 //                inverse, real and imaginary parts are the two real rows (c2r)
 //   k_fxy3_r2c : for N <= 144 the x and y forward passes of one plane in one block
@@ -181,8 +183,8 @@ __device__ __forceinline__ void seq_transform_g(float2* base, int se, int t, con
 // Mesh layouts (both in place, potential written over the input):
 //  row-pitched (five-pass sizes): row pitch RP bytes = max(N*rb, (N/2+1)*8) up to 16, so a real
 //    row and its half-spectrum row share bytes (FFTW's in-place r2c layout); plane = N rows;
-//  plane-compact (fused sizes): real rows of N, half-spectrum rows of N/2+1 and phi rows of
-//    N packed from the start of each plane; plane pitch max(N*N*rb, N*(N/2+1)*8) bytes.
+//  plane-compact (fused sizes): real rows of N, half-spectrum rows of N/2+1 up to even and phi
+//    rows of N packed from the start of each plane; plane pitch the larger of the two.
 // Kernels take the row pitch (pr real elements, pc complex, pf floats) and the plane pitch
 // in the same units (plr, plc, plf).
 
@@ -232,20 +234,28 @@ __global__ void __launch_bounds__(256) k_fx_r2c(const IN* r, float2* c, int64_t 
 // one shared-memory exchange, then thread t = k1 runs the R2-point DFT and holds
 // X[t + R1*k2].  The inverse uses the swapped factorisation (n = R1*n1 + n2), whose
 // first step needs in thread t exactly the X[t + R1*k2] it already holds, so
-// forward -> Green multiply -> inverse costs two exchanges in all.
-//   MODE 0: forward, 1: inverse, 2: forward -> multiply by green[kz][y][kx] -> inverse.
-// Shared memory: tw[N], exchange slots [N][W] float2, and for MODE 2 the column's Green
-// values [N][W] float, prefetched with cp.async at the start.
+// forward -> Green multiply -> inverse (k_fz_loop, k_fz_stream) costs two exchanges in all.
+//   MODE 0: forward, 1: inverse.
+// Shared memory: tw[N], exchange slots [N][W] float2.
 // ---------------------------------------------------------------------------------
-// Launch bounds of the column pass: two blocks per SM where the sequences fit in 64
-// registers (or 73 with the 444-thread blocks of N = 144), one block above N = 192.
-template <int N>
+// Column-block width: the whole half row when it fits one block, else an even split.
+constexpr int fcol_width(int N, int T) {
+  const int NH = N / 2 + 1, maxt = N == 144 ? 448 : 512;
+  for (int nb = 1;; ++nb) {
+    const int W = (NH + nb - 1) / nb;
+    if (W * T <= maxt && W * N * 8 <= 100 * 1024) return W;
+  }
+}
+// Launch bounds of the column pass: the block's own threads, two blocks per SM up to N = 288
+// (64 or 72 registers; one block, as the bound of 512 threads left it, kept half of the SM's
+// warps idle: the two y passes of eight 288^3 meshes took 1.06 ms).
+template <int N, int T>
 struct FcolBounds {
-  static constexpr int MAXT = (N == 144) ? 448 : 512, MINB = (N <= 192) ? 2 : 1;
+  static constexpr int MAXT = (fcol_width(N, T) * T + 31) / 32 * 32, MINB = (N <= 288) ? 2 : 1;
 };
 
 template <int N, int R1, int R2, int AXIS, int MODE>
-__global__ void __launch_bounds__(FcolBounds<N>::MAXT, FcolBounds<N>::MINB) k_fcol3(float2* __restrict__ c, const float* __restrict__ green,
+__global__ void __launch_bounds__(FcolBounds<N, TPS<R1, R2>::T>::MAXT, FcolBounds<N, TPS<R1, R2>::T>::MINB) k_fcol3(float2* __restrict__ c,
                                                   const float2* __restrict__ gtw, int W, int pc, int64_t plc) {
   constexpr int NH = N / 2 + 1;
   extern __shared__ float2 sm[];
@@ -261,15 +271,6 @@ __global__ void __launch_bounds__(FcolBounds<N>::MAXT, FcolBounds<N>::MINB) k_fc
   const int64_t es = (AXIS == 1) ? pc : plc;
   float2* base = c + b * (int64_t)N * plc + (AXIS == 1 ? (int64_t)o * plc : (int64_t)o * pc) + kx0 + col;
   float2* Ac = A + col;
-  float* Gc = reinterpret_cast<float*>(A + (size_t)N * W) + col;  // MODE 2: green[kz] of this column, [N][W]
-  if (MODE == 2) {
-    if (t < R1 && live) {
-      const float* gb = green + (int64_t)o * NH + kx0 + col;  // g[kz][y][kx]
-#pragma unroll
-      for (int k2 = 0; k2 < R2; ++k2) cp_async4(Gc + (t + R1 * k2) * W, gb + (int64_t)(t + R1 * k2) * N * NH);
-    }
-    cp_async_commit();
-  }
   __syncthreads();
   if (MODE != 1) {
     // ---- forward: n = R2*n1 + n2 ----
@@ -288,43 +289,9 @@ __global__ void __launch_bounds__(FcolBounds<N>::MAXT, FcolBounds<N>::MINB) k_fc
       for (int n2 = 0; n2 < R2; ++n2) w[n2] = Ac[(t * R2 + n2) * W];
       DFT<R2, N, -1>::run(w, tw);
     }
-    if (MODE == 0) {
-      if (t < R1 && live) {
-#pragma unroll
-        for (int k2 = 0; k2 < R2; ++k2) base[(int64_t)(t + R1 * k2) * es] = w[k2];
-      }
-      return;
-    }
-    // ---- Green multiply at kz = t + R1*k2 (values this thread prefetched) ----
-    cp_async_wait_all();
     if (t < R1 && live) {
 #pragma unroll
-      for (int k2 = 0; k2 < R2; ++k2) {
-        const float gv = Gc[(t + R1 * k2) * W];
-        w[k2] = make_float2(w[k2].x * gv, w[k2].y * gv);
-      }
-    }
-    // ---- inverse, n = R1*n1 + n2 with n2 = t, n1 = k2: first step in registers ----
-    if (t < R1) {
-      DFT<R2, N, +1>::run(w, tw);
-#pragma unroll
-      for (int k1 = 1; k1 < R2; ++k1) w[k1] = cmul(w[k1], twid<+1>(tw, t * k1));
-    }
-    __syncthreads();  // every forward read of the slots is done
-    if (t < R1) {
-#pragma unroll
-      for (int k1 = 0; k1 < R2; ++k1) Ac[(k1 * R1 + t) * W] = w[k1];
-    }
-    __syncthreads();
-    if (t < R2) {
-      float2 u[R1];
-#pragma unroll
-      for (int n2 = 0; n2 < R1; ++n2) u[n2] = Ac[(t * R1 + n2) * W];
-      DFT<R1, N, +1>::run(u, tw);
-      if (live) {
-#pragma unroll
-        for (int k2 = 0; k2 < R1; ++k2) base[(int64_t)(t + R2 * k2) * es] = u[k2];
-      }
+      for (int k2 = 0; k2 < R2; ++k2) base[(int64_t)(t + R1 * k2) * es] = w[k2];
     }
   } else {
     // ---- inverse only, n = R1*n1 + n2: thread t = n2 < R1 loads x[R1*n1 + t] ----
@@ -351,7 +318,125 @@ __global__ void __launch_bounds__(FcolBounds<N>::MAXT, FcolBounds<N>::MINB) k_fc
 }
 
 // ---------------------------------------------------------------------------------
-// Persistent z pass with Green multiply: the work of k_fcol3<...,2,2> (forward z DFT,
+// z pass with Green multiply for the plane sizes (N <= 144): forward z DFT, Green multiply,
+// inverse, with a block kept on one line y and one group of columns while it walks the boxes, so the
+// group's Green values are read once, and the next box's columns are copied into the other
+// of two shared-memory stages (16-byte copies) while the current one is transformed.  A
+// stage doubles as the exchange: the first step writes the slots it read.  Four barriers a
+// box.  One line per block, loaded when the block starts, two blocks per SM, left
+// the loads exposed: 4.63 ms for 512 boxes of 144^3, 3.1 ms now (1.9 at the copy bandwidth).
+// Column groups start at even columns, for the 16-byte copies; the row pitch is even.
+// ---------------------------------------------------------------------------------
+template <int N, int R1, int R2>
+struct ZLoop {
+  static constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1;
+  static constexpr int NCG = (NH * T + 447) / 448;
+  static constexpr int STEP = NCG == 1 ? NH : (NH + NCG - 1) / NCG / 2 * 2;  // columns between groups
+  static constexpr int LAST = NH - STEP * (NCG - 1), COLS = LAST > STEP ? LAST : STEP;
+  static constexpr int WC = (COLS + 1) / 2 * 2;  // columns copied
+  static_assert(STEP * (NCG - 1) + WC <= (NH + 1) / 2 * 2, "copies stay in the row");
+  static constexpr int THREADS = (COLS * T + 31) / 32 * 32;
+  static constexpr int MINB = N == 96 ? 3 : N >= 96 ? 2 : N >= 64 ? 4 : N >= 48 ? 6 : 8;
+  static constexpr size_t SMEM = (size_t)N * 8 + (size_t)2 * N * WC * 8 + (size_t)N * COLS * 4;
+};
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
+template <int N, int R1, int R2>
+__global__ void __launch_bounds__(ZLoop<N, R1, R2>::THREADS, ZLoop<N, R1, R2>::MINB)
+    k_fz_loop(float2* __restrict__ c, const float* __restrict__ green, const float2* __restrict__ gtw, int pc, int64_t plc,
+              int64_t nbox, int nsplit) {
+  using Z = ZLoop<N, R1, R2>;
+  constexpr int NH = Z::NH, WC = Z::WC, COLS = Z::COLS;
+  extern __shared__ __align__(16) float2 sm[];
+  float2* const stg = sm;                                             // [2][N][WC]
+  float2* const tw = sm + 2 * N * WC;                                 // [N]
+  float* const gr = reinterpret_cast<float*>(tw + N);                 // [N][COLS]
+  const int line = blockIdx.x / nsplit, y = line / Z::NCG, g = line - y * Z::NCG, kx0 = g * Z::STEP;
+  const int ncol = g == Z::NCG - 1 ? Z::LAST : Z::STEP;
+  const int col = threadIdx.x % COLS, t = threadIdx.x / COLS;
+  const bool live = col < ncol;
+  for (int i = threadIdx.x; i < N; i += Z::THREADS) tw[i] = gtw[i];
+  for (int i = threadIdx.x; i < N * COLS; i += Z::THREADS) {
+    const int z = i / COLS, q = i - z * COLS;
+    gr[i] = q < ncol ? green[((int64_t)z * N + y) * NH + kx0 + q] : 0.f;
+  }
+  auto base = [&](int64_t b) { return c + b * (int64_t)N * plc + (int64_t)y * pc + kx0; };
+  auto issue = [&](int64_t b, int st) {
+    const float2* src = base(b);
+    float2* dst = stg + st * N * WC;
+    for (int i = threadIdx.x; i < N * (WC / 2); i += Z::THREADS) {
+      const int z = i / (WC / 2), q = 2 * (i - z * (WC / 2));
+      cp_async16(dst + z * WC + q, src + (int64_t)z * plc + q);
+    }
+  };
+  int64_t b = blockIdx.x - (int64_t)line * nsplit;
+  if (b < nbox) issue(b, 0);
+  cp_async_commit();
+  for (int st = 0; b < nbox; b += nsplit, st ^= 1) {
+    cp_async_wait_all();
+    __syncthreads();  // the box's columns are in; the other stage is free
+    if (b + nsplit < nbox) issue(b + nsplit, st ^ 1);
+    cp_async_commit();
+    float2* const A = stg + st * N * WC + col;
+    if (t < R2) {  // forward, n = R2*n1 + n2, thread t = n2
+      float2 v[R1];
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) v[n1] = A[(R2 * n1 + t) * WC];
+      DFT<R1, N, -1>::run(v, tw);
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) A[(k1 * R2 + t) * WC] = (k1 == 0) ? v[0] : cmul(v[k1], twid<-1>(tw, t * k1));
+    }
+    __syncthreads();
+    float2 w[R2];
+    if (t < R1) {
+#pragma unroll
+      for (int n2 = 0; n2 < R2; ++n2) w[n2] = A[(t * R2 + n2) * WC];
+      DFT<R2, N, -1>::run(w, tw);
+#pragma unroll
+      for (int k2 = 0; k2 < R2; ++k2) {  // Green at kz = t + R1*k2
+        const float gv = gr[(t + R1 * k2) * COLS + col];
+        w[k2] = make_float2(w[k2].x * gv, w[k2].y * gv);
+      }
+      // inverse, n = R1*n1 + n2 with n2 = t, n1 = k2
+      DFT<R2, N, +1>::run(w, tw);
+#pragma unroll
+      for (int k1 = 1; k1 < R2; ++k1) w[k1] = cmul(w[k1], twid<+1>(tw, t * k1));
+    }
+    __syncthreads();
+    if (t < R1) {
+#pragma unroll
+      for (int k1 = 0; k1 < R2; ++k1) A[(k1 * R1 + t) * WC] = w[k1];
+    }
+    __syncthreads();
+    if (t < R2) {
+      float2 u[R1];
+#pragma unroll
+      for (int n2 = 0; n2 < R1; ++n2) u[n2] = A[(t * R1 + n2) * WC];
+      DFT<R1, N, +1>::run(u, tw);
+      if (live) {
+        float2* out = base(b) + col;
+#pragma unroll
+        for (int k2 = 0; k2 < R1; ++k2) out[(int64_t)(t + R2 * k2) * plc] = u[k2];
+      }
+    }
+  }
+}
+
+// Blocks per line of k_fz_loop: enough to fill the chip once, and else about 24 boxes a block,
+// which hides a block's start (its Green values, the first copy) and still deals the boxes
+// out evenly (512 boxes of 144^3: 3.28 ms with one block a line, 3.14 so; 64 boxes: 0.74 ms
+// with a box a block, 0.43 so).
+inline int fz_loop_split(int lines, int resident, int64_t nbox) {
+  const int64_t s = std::max<int64_t>(std::min<int64_t>(nbox, resident / lines), nbox / 24);
+  return (int)std::max<int64_t>(1, s);
+}
+
+// ---------------------------------------------------------------------------------
+// Persistent z pass with Green multiply for N > 144 (forward z DFT,
 // Green multiply, inverse), one item = W columns of one line (box b, row y), looped over
 // by a grid of a few blocks per SM.  The column data and Green values of the next item
 // are copied into the other of two shared-memory stages with cp.async while the current
@@ -471,17 +556,6 @@ __host__ inline void fz_stream_shape(int N, int T, int& W, int& ncg) {
   W = (NH + ncg - 1) / ncg;
 }
 __host__ inline size_t fz_stream_smem(int N, int W) { return (size_t)N * 8 + (size_t)2 * N * W * 12; }
-
-// Column-block width: the whole half row when it fits one block (<= 512 threads, the
-// launch bound), else an even split.
-__host__ inline int fcol_width(int N, int T) {
-  const int NH = N / 2 + 1;
-  const int maxt = (N == 144) ? 448 : 512;  // FcolBounds<N>::MAXT
-  for (int nb = 1;; ++nb) {
-    const int W = (NH + nb - 1) / nb;
-    if (W * T <= maxt && (size_t)W * N * 8 <= 100 * 1024) return W;
-  }
-}
 
 // ---------------------------------------------------------------------------------
 // X' pass, c2r, divided `reps` times by `norm`.  In place (complex rows pc -> real rows pf).

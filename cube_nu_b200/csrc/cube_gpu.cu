@@ -1405,10 +1405,8 @@ static int enqueue_kick_a(cube_ctx* c) {
     const int n = G.nc;
     MeshPtrs m = mesh_ptrs(c, n, 1, fixed);
     CK(cudaMemsetAsync(m.real, 0, mesh_bytes(c, n, 1, fixed), c->s));
-    if (fixed)
-      LAUNCH(c, K_DEP_PM1, 1, k_deposit_pm1_runs<<<nblk(npo), 256, 0, c->s>>>(G, npo, xpo, pco,
-                                                                     reinterpret_cast<unsigned long long*>(m.real), m.pt.pr, m.pt.plr, ms1));
-    else LAUNCH(c, K_DEP_PM1, 1, k_deposit_pm1<false><<<nblk(npo), 256, 0, c->s>>>(G, npo, xpo, pco, m.real, m.pt.pr, m.pt.plr, ms1));
+    auto kd1 = fixed ? k_deposit_pm1<true> : k_deposit_pm1<false>;
+    LAUNCH(c, K_DEP_PM1, 1, kd1<<<nblk(npo), 256, 0, c->s>>>(G, npo, xpo, pco, m.real, m.pt.pr, m.pt.plr, ms1));
     if (G.nslab > 1) {
       const int64_t nel = (int64_t)(mesh_bytes(c, n, 1, fixed) / (fixed ? 8 : 4));
       const int rc = comm_allreduce(c, m.real, nel, fixed ? CUBE_DT_I64 : CUBE_DT_F32, CUBE_OP_SUM, 1);

@@ -144,6 +144,13 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
       : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
   return reinterpret_cast<const float2&>(r);
 }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return reinterpret_cast<const float2&>(r);
+}
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   unsigned long long r;
   asm("mul.rn.f32x2 %0, %1, %2;"

@@ -17,6 +17,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace cube {
 
 struct FFTDesc {
@@ -29,8 +31,8 @@ struct FFTDesc {
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return add2(a, b); }  // one packed instruction
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return sub2(a, b); }
 
 // Batched Stockham FFT in shared memory.  Sequence s, element e at
 // buf[s*sb + e*se].  SFAST selects the thread mapping (sequence index fastest when

@@ -5,8 +5,8 @@
 //   step 1 (thread n2): R1-point DFT over n1, times w_N^(n2*k1), written in place;
 //   step 2 (thread k1): R2-point DFT over n2, written to k1 + R1*k2.
 // The R-point DFTs are unrolled in registers, composed recursively from radix 2/3/4
-// with inner twiddles read at compile-time indices of a shared table
-// tw[j] = e^{-2 pi i j/N} (built on the host in double precision).  With N a template
+// with inner twiddles that are compile-time constants; the twiddles between the steps come
+// from a shared table tw[j] = e^{-2 pi i j/N} (built on the host in double precision).  With N a template
 // parameter every index is strength-reduced; no runtime integer division remains in
 // the butterflies.
 //
@@ -54,29 +54,74 @@ struct Split {
   static constexpr int B = R / A;
 };
 
-// R-point DFT in registers (sign DIR); inner twiddles from the N-point table.
+// cos and sin of 2 pi j / n at compile time (Taylor series in double, |angle| <= pi).
+constexpr double ct_pi = 3.14159265358979323846;
+__host__ __device__ constexpr double ct_series(double x, double term, int k) {  // sum of (-1)^i x^(2i+k) / (2i+k)!
+  double s = 0.0;
+  for (int i = 0; i < 24; ++i) {
+    s += term;
+    term *= -x * x / ((2 * i + k + 1) * (2 * i + k + 2));
+  }
+  return s;
+}
+__host__ __device__ constexpr double ct_angle(int j, int n) { return 2.0 * ct_pi * (2 * j > n ? j - n : j) / n; }
+__host__ __device__ constexpr double ct_cos(int j, int n) { return ct_series(ct_angle(j, n), 1.0, 0); }
+__host__ __device__ constexpr double ct_sin(int j, int n) { return ct_series(ct_angle(j, n), ct_angle(j, n), 1); }
+
+template <int I>
+struct Int {
+  static constexpr int v = I;
+};
+template <int I, int N, class F>
+__device__ __forceinline__ void static_for(F&& f) {
+  if constexpr (I < N) {
+    f(Int<I>{});
+    static_for<I + 1, N>(f);
+  }
+}
+
+// u times e^{DIR 2 pi i J / R}, the constant an immediate operand; nothing but a swap for
+// multiples of a quarter turn.
+template <int R, int J, int DIR>
+__device__ __forceinline__ float2 ct_twiddle(float2 u) {
+  if constexpr (J == 0) return u;
+  else if constexpr (2 * J == R) return make_float2(-u.x, -u.y);
+  else if constexpr (4 * J == R || 4 * J == 3 * R) {
+    constexpr bool plus = (4 * J == R) == (DIR > 0);  // times +i or -i
+    return plus ? make_float2(-u.y, u.x) : make_float2(u.y, -u.x);
+  } else {
+    constexpr float c = (float)ct_cos(J, R), s = (float)(DIR * ct_sin(J, R));
+    return make_float2(u.x * c - u.y * s, u.x * s + u.y * c);
+  }
+}
+
+// R-point DFT in registers (sign DIR).  Sums and differences are packed, two components to
+// an instruction, and the inner twiddles are constants: a 12-point transform takes 78
+// floating-point instructions and no reads of the twiddle table, 128 and 6 without either
+// (512 boxes of 144^3: 4.13 + 3.32 + 4.01 ms for the three passes, 3.86 + 3.10 + 3.86 with).
 template <int R, int N, int DIR>
 struct DFT {
   static constexpr int A = Split<R>::A, B = Split<R>::B;
   static_assert(N % R == 0, "DFT size must divide the table size");
-  __device__ __forceinline__ static void run(float2* v, const float2* tw) {
+  __device__ __forceinline__ static void run(float2* v) {
     float2 tmp[R];
-#pragma unroll
-    for (int n2 = 0; n2 < B; ++n2) {
+    static_for<0, B>([&](auto i2) {
+      constexpr int n2 = decltype(i2)::v;
       float2 u[A];
 #pragma unroll
       for (int n1 = 0; n1 < A; ++n1) u[n1] = v[B * n1 + n2];
-      DFT<A, N, DIR>::run(u, tw);
-#pragma unroll
-      for (int k1 = 0; k1 < A; ++k1)
-        tmp[k1 * B + n2] = (n2 * k1 == 0) ? u[k1] : cmul(u[k1], twid<DIR>(tw, ((n2 * k1) % R) * (N / R)));
-    }
+      DFT<A, N, DIR>::run(u);
+      static_for<0, A>([&](auto i1) {
+        constexpr int k1 = decltype(i1)::v;
+        tmp[k1 * B + n2] = ct_twiddle<R, (n2 * k1) % R, DIR>(u[k1]);
+      });
+    });
 #pragma unroll
     for (int k1 = 0; k1 < A; ++k1) {
       float2 w[B];
 #pragma unroll
       for (int n2 = 0; n2 < B; ++n2) w[n2] = tmp[k1 * B + n2];
-      DFT<B, N, DIR>::run(w, tw);
+      DFT<B, N, DIR>::run(w);
 #pragma unroll
       for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = w[k2];
     }
@@ -85,12 +130,12 @@ struct DFT {
 
 template <int N, int DIR>
 struct DFT<1, N, DIR> {
-  __device__ __forceinline__ static void run(float2*, const float2*) {}
+  __device__ __forceinline__ static void run(float2*) {}
 };
 
 template <int N, int DIR>
 struct DFT<2, N, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2*) {
+  __device__ __forceinline__ static void run(float2* v) {
     const float2 a = v[0], b = v[1];
     v[0] = cadd(a, b);
     v[1] = csub(a, b);
@@ -99,21 +144,20 @@ struct DFT<2, N, DIR> {
 
 template <int N, int DIR>
 struct DFT<3, N, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2*) {
+  __device__ __forceinline__ static void run(float2* v) {
     const float s3 = 0.8660254037844386f * (float)DIR;
     const float2 t1 = cadd(v[1], v[2]);
     const float2 d = csub(v[1], v[2]);
-    const float2 m0 = make_float2(v[0].x - 0.5f * t1.x, v[0].y - 0.5f * t1.y);
-    const float2 id = make_float2(-d.y * s3, d.x * s3);
+    const float2 m0 = fma2(make_float2(-0.5f, -0.5f), t1, v[0]);
     v[0] = cadd(v[0], t1);
-    v[1] = cadd(m0, id);
-    v[2] = csub(m0, id);
+    v[1] = make_float2(fmaf(-d.y, s3, m0.x), fmaf(d.x, s3, m0.y));
+    v[2] = make_float2(fmaf(d.y, s3, m0.x), fmaf(-d.x, s3, m0.y));
   }
 };
 
 template <int N, int DIR>
 struct DFT<4, N, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2*) {
+  __device__ __forceinline__ static void run(float2* v) {
     const float2 a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]);
     const float2 b0 = cadd(v[1], v[3]), b1 = csub(v[1], v[3]);
     const float2 jb1 = (DIR < 0) ? make_float2(b1.y, -b1.x) : make_float2(-b1.y, b1.x);
@@ -132,14 +176,14 @@ struct Seq {
     float2 v[R1];
 #pragma unroll
     for (int n1 = 0; n1 < R1; ++n1) v[n1] = base[(R2 * n1 + t) * se];
-    DFT<R1, N, DIR>::run(v, tw);
+    DFT<R1, N, DIR>::run(v);
 #pragma unroll
     for (int k1 = 0; k1 < R1; ++k1) base[(R2 * k1 + t) * se] = (k1 == 0) ? v[0] : cmul(v[k1], twid<DIR>(tw, t * k1));
   }
   __device__ __forceinline__ static void step2_load(const float2* base, int se, int t, float2* w, const float2* tw) {
 #pragma unroll
     for (int n2 = 0; n2 < R2; ++n2) w[n2] = base[(R2 * t + n2) * se];
-    DFT<R2, N, DIR>::run(w, tw);
+    DFT<R2, N, DIR>::run(w);
   }
   __device__ __forceinline__ static void step2_store(float2* base, int se, int t, const float2* w) {
 #pragma unroll
@@ -278,7 +322,7 @@ __global__ void __launch_bounds__(FcolBounds<N, TPS<R1, R2>::T>::MAXT, FcolBound
       float2 v[R1];
 #pragma unroll
       for (int n1 = 0; n1 < R1; ++n1) v[n1] = live ? base[(int64_t)(R2 * n1 + t) * es] : make_float2(0.f, 0.f);
-      DFT<R1, N, -1>::run(v, tw);
+      DFT<R1, N, -1>::run(v);
 #pragma unroll
       for (int k1 = 0; k1 < R1; ++k1) Ac[(k1 * R2 + t) * W] = (k1 == 0) ? v[0] : cmul(v[k1], twid<-1>(tw, t * k1));
     }
@@ -287,7 +331,7 @@ __global__ void __launch_bounds__(FcolBounds<N, TPS<R1, R2>::T>::MAXT, FcolBound
     if (t < R1) {
 #pragma unroll
       for (int n2 = 0; n2 < R2; ++n2) w[n2] = Ac[(t * R2 + n2) * W];
-      DFT<R2, N, -1>::run(w, tw);
+      DFT<R2, N, -1>::run(w);
     }
     if (t < R1 && live) {
 #pragma unroll
@@ -299,7 +343,7 @@ __global__ void __launch_bounds__(FcolBounds<N, TPS<R1, R2>::T>::MAXT, FcolBound
       float2 w[R2];
 #pragma unroll
       for (int n1 = 0; n1 < R2; ++n1) w[n1] = live ? base[(int64_t)(R1 * n1 + t) * es] : make_float2(0.f, 0.f);
-      DFT<R2, N, +1>::run(w, tw);
+      DFT<R2, N, +1>::run(w);
 #pragma unroll
       for (int k1 = 0; k1 < R2; ++k1) Ac[(k1 * R1 + t) * W] = (k1 == 0) ? w[0] : cmul(w[k1], twid<+1>(tw, t * k1));
     }
@@ -308,7 +352,7 @@ __global__ void __launch_bounds__(FcolBounds<N, TPS<R1, R2>::T>::MAXT, FcolBound
       float2 u[R1];
 #pragma unroll
       for (int n2 = 0; n2 < R1; ++n2) u[n2] = Ac[(t * R1 + n2) * W];
-      DFT<R1, N, +1>::run(u, tw);
+      DFT<R1, N, +1>::run(u);
       if (live) {
 #pragma unroll
         for (int k2 = 0; k2 < R1; ++k2) base[(int64_t)(t + R2 * k2) * es] = u[k2];
@@ -386,7 +430,7 @@ __global__ void __launch_bounds__(ZLoop<N, R1, R2>::THREADS, ZLoop<N, R1, R2>::M
       float2 v[R1];
 #pragma unroll
       for (int n1 = 0; n1 < R1; ++n1) v[n1] = A[(R2 * n1 + t) * WC];
-      DFT<R1, N, -1>::run(v, tw);
+      DFT<R1, N, -1>::run(v);
 #pragma unroll
       for (int k1 = 0; k1 < R1; ++k1) A[(k1 * R2 + t) * WC] = (k1 == 0) ? v[0] : cmul(v[k1], twid<-1>(tw, t * k1));
     }
@@ -395,14 +439,14 @@ __global__ void __launch_bounds__(ZLoop<N, R1, R2>::THREADS, ZLoop<N, R1, R2>::M
     if (t < R1) {
 #pragma unroll
       for (int n2 = 0; n2 < R2; ++n2) w[n2] = A[(t * R2 + n2) * WC];
-      DFT<R2, N, -1>::run(w, tw);
+      DFT<R2, N, -1>::run(w);
 #pragma unroll
       for (int k2 = 0; k2 < R2; ++k2) {  // Green at kz = t + R1*k2
         const float gv = gr[(t + R1 * k2) * COLS + col];
         w[k2] = make_float2(w[k2].x * gv, w[k2].y * gv);
       }
       // inverse, n = R1*n1 + n2 with n2 = t, n1 = k2
-      DFT<R2, N, +1>::run(w, tw);
+      DFT<R2, N, +1>::run(w);
 #pragma unroll
       for (int k1 = 1; k1 < R2; ++k1) w[k1] = cmul(w[k1], twid<+1>(tw, t * k1));
     }
@@ -416,7 +460,7 @@ __global__ void __launch_bounds__(ZLoop<N, R1, R2>::THREADS, ZLoop<N, R1, R2>::M
       float2 u[R1];
 #pragma unroll
       for (int n2 = 0; n2 < R1; ++n2) u[n2] = A[(t * R1 + n2) * WC];
-      DFT<R1, N, +1>::run(u, tw);
+      DFT<R1, N, +1>::run(u);
       if (live) {
         float2* out = base(b) + col;
 #pragma unroll
@@ -502,7 +546,7 @@ __global__ void __launch_bounds__(fzs_maxt(N), (N <= 192 ? 2 : 1)) k_fz_stream(f
     if (thr && t < R2) {
 #pragma unroll
       for (int n1 = 0; n1 < R1; ++n1) v[n1] = live ? Ac[(R2 * n1 + t) * W] : make_float2(0.f, 0.f);
-      DFT<R1, N, -1>::run(v, tw);
+      DFT<R1, N, -1>::run(v);
     }
     __syncthreads();  // the stage's data are in registers; its slots become the exchange
     if (thr && t < R2) {
@@ -514,14 +558,14 @@ __global__ void __launch_bounds__(fzs_maxt(N), (N <= 192 ? 2 : 1)) k_fz_stream(f
     if (thr && t < R1) {
 #pragma unroll
       for (int n2 = 0; n2 < R2; ++n2) w[n2] = Ac[(t * R2 + n2) * W];
-      DFT<R2, N, -1>::run(w, tw);
+      DFT<R2, N, -1>::run(w);
 #pragma unroll
       for (int k2 = 0; k2 < R2; ++k2) {  // Green at kz = t + R1*k2
         const float gv = Gc[(t + R1 * k2) * W];
         w[k2] = make_float2(w[k2].x * gv, w[k2].y * gv);
       }
       // inverse, n = R1*n1 + n2 with n2 = t, n1 = k2
-      DFT<R2, N, +1>::run(w, tw);
+      DFT<R2, N, +1>::run(w);
 #pragma unroll
       for (int k1 = 1; k1 < R2; ++k1) w[k1] = cmul(w[k1], twid<+1>(tw, t * k1));
     }
@@ -535,7 +579,7 @@ __global__ void __launch_bounds__(fzs_maxt(N), (N <= 192 ? 2 : 1)) k_fz_stream(f
       float2 u[R1];
 #pragma unroll
       for (int n2 = 0; n2 < R1; ++n2) u[n2] = Ac[(t * R1 + n2) * W];
-      DFT<R1, N, +1>::run(u, tw);
+      DFT<R1, N, +1>::run(u);
       if (live) {
 #pragma unroll
         for (int k2 = 0; k2 < R1; ++k2) out[(int64_t)(t + R2 * k2) * plc] = u[k2];
@@ -674,7 +718,7 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
           }
           v[n1] = make_float2(__fmul_rn(fa, scale), __fmul_rn(fb, scale));
         }
-        DFT<R1, N, -1>::run(v, tw);
+        DFT<R1, N, -1>::run(v);
 #pragma unroll
         for (int k1 = 0; k1 < R1; ++k1) Zr[skew<R1, R2>(k1, t)] = (k1 == 0) ? v[0] : cmul(v[k1], twid<-1>(tw, t * k1));
       }
@@ -683,7 +727,7 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
       if (act && t < R1) {
 #pragma unroll
         for (int n2 = 0; n2 < R2; ++n2) w[n2] = Zr[skew<R1, R2>(t, n2)];
-        DFT<R2, N, -1>::run(w, tw);
+        DFT<R2, N, -1>::run(w);
       }
       __syncwarp();
       if (act && t < R1) {
@@ -719,7 +763,7 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
           v[n1] = (y & 1) ? make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x))
                           : make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
         }
-        DFT<R1, N, -1>::run(v, tw);
+        DFT<R1, N, -1>::run(v);
       }
       __syncthreads();  // all unpack reads of this round are done
       if (act && t < R2) {
@@ -742,7 +786,7 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
           const int sl = s0 + n2;
           w[n2] = Z[(whole ? b : (sl < NP ? lo : hi)) + (int64_t)sl * st];
         }
-        DFT<R2, N, -1>::run(w, tw);
+        DFT<R2, N, -1>::run(w);
 #pragma unroll
         for (int k2 = 0; k2 < R2; ++k2) cp[(int64_t)(t + R1 * k2) * pc + kx] = w[k2];
       }
@@ -775,7 +819,7 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
         float2 v[R1];
 #pragma unroll
         for (int n1 = 0; n1 < R1; ++n1) v[n1] = cp[(int64_t)(R2 * n1 + t) * pc + kx];
-        DFT<R1, N, +1>::run(v, tw);
+        DFT<R1, N, +1>::run(v);
 #pragma unroll
         for (int k1 = 0; k1 < R1; ++k1) Hc[(k1 * R2 + t) * NH] = (k1 == 0) ? v[0] : cmul(v[k1], twid<+1>(tw, t * k1));
       }
@@ -784,7 +828,7 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
       if (act && t < R1) {
 #pragma unroll
         for (int n2 = 0; n2 < R2; ++n2) w[n2] = Hc[(t * R2 + n2) * NH];
-        DFT<R2, N, +1>::run(w, tw);
+        DFT<R2, N, +1>::run(w);
       }
       __syncthreads();  // every read of the column's slots is done
       if (act && t < R1) {
@@ -821,7 +865,7 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
           }
           v[n1] = make_float2(a0.x - a1.y, a0.y + a1.x);
         }
-        DFT<R1, N, +1>::run(v, tw);
+        DFT<R1, N, +1>::run(v);
       }
       __syncwarp();  // the pack reads of rows 2p, 2p+1 are done
       if (act && t < R2) {
@@ -833,7 +877,7 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
         float2 w[R2];
 #pragma unroll
         for (int n2 = 0; n2 < R2; ++n2) w[n2] = H0[skew<R1, R2>(t, n2)];
-        DFT<R2, N, +1>::run(w, tw);
+        DFT<R2, N, +1>::run(w);
 #pragma unroll
         for (int k2 = 0; k2 < R2; ++k2) {
           const int x = t + R1 * k2;

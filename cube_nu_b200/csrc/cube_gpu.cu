@@ -500,7 +500,7 @@ void fz_green(cube_ctx* c, int64_t nbox, float2* ck, const float* green, const f
 
 template <int N, int R1, int R2>
 void fft2_run(cube_ctx* c, int64_t nbox, const void* real_in, bool fixed, float scale, float* phi_out, float2* ck,
-              const float* green, float inv, int kx, int ky, int kz, int kc, const Pitch& pt) {
+              const float* green, float inv, int kx, int ky, int kz, int kc, const Pitch& pt, int lo, int hi) {
   constexpr int T = f2::TPS<R1, R2>::T, NH = N / 2 + 1;
   const float2* tw = fft_desc(c, N)->tw;
   const int64_t nrows = nbox * (int64_t)N * N;
@@ -524,10 +524,12 @@ void fft2_run(cube_ctx* c, int64_t nbox, const void* real_in, bool fixed, float 
       const int lines = N * Z::NCG, ns = f2::fz_loop_split(lines, c->nsm * Z::MINB, nbox);
       auto zl = f2::k_fz_loop<N, R1, R2>;
       smem_optin(zl, Z::SMEM);
-      LAUNCH(c, kz, 1, zl<<<(unsigned)(lines * ns), Z::THREADS, Z::SMEM, c->s>>>(ck, green, tw, pt.pc, pt.plc, nbox, ns));
+      LAUNCH(c, kz, 1, zl<<<(unsigned)(lines * ns), Z::THREADS, Z::SMEM, c->s>>>(ck, green, tw, pt.pc, pt.plc, nbox, ns, lo,
+                                                                                 hi));
       smem_optin(f2::k_fyx3_c2r<N, R1, R2>, smi);
-      LAUNCH(c, kc, 1, f2::k_fyx3_c2r<N, R1, R2><<<planes, f2::PlaneShape<N, R1, R2>::THREADS, smi, c->s>>>(
-                           ck, phi_out, tw, inv, pt.pc, pt.pf, pt.plc, pt.plf));
+      const unsigned cplanes = (unsigned)(nbox * (hi - lo));
+      LAUNCH(c, kc, 1, f2::k_fyx3_c2r<N, R1, R2><<<cplanes, f2::PlaneShape<N, R1, R2>::THREADS, smi, c->s>>>(
+                           ck, phi_out, tw, inv, pt.pc, pt.pf, pt.plc, pt.plf, lo, hi));
       return;
     }
   }
@@ -565,9 +567,9 @@ bool fft2_size(int n) {
 bool fused_layout(const cube_ctx* c, int n) { return !c->fft_generic && c->fft_fused && n <= 144 && fft2_size(n); }
 
 bool fft2_dispatch(cube_ctx* c, int n, int64_t nbox, const void* real_in, bool fixed, float scale, float* phi_out,
-                   float2* ck, const float* green, float inv, int kx, int ky, int kz, int kc, const Pitch& pt) {
+                   float2* ck, const float* green, float inv, int kx, int ky, int kz, int kc, const Pitch& pt, int lo, int hi) {
 #define CUBE_FFT2(N, R1, R2) \
-  case N: fft2_run<N, R1, R2>(c, nbox, real_in, fixed, scale, phi_out, ck, green, inv, kx, ky, kz, kc, pt); return true;
+  case N: fft2_run<N, R1, R2>(c, nbox, real_in, fixed, scale, phi_out, ck, green, inv, kx, ky, kz, kc, pt, lo, hi); return true;
   switch (n) {
     CUBE_FFT2(16, 4, 4)
     CUBE_FFT2(32, 4, 8)
@@ -663,8 +665,10 @@ bool fft2_forward_dispatch(cube_ctx* c, int n, float* real, const Pitch& pt, int
 #undef CUBE_FFT2F
 }
 
+// lo, hi: the potential is wanted in array cells [lo, hi) of each dimension at least (the whole
+// mesh without them); the plane sizes leave the rest out.
 void launch_fft(cube_ctx* c, int n, int64_t nbox, const void* real_in, bool fixed, float scale, float* phi_out,
-                float2* ck, const float* green, float norm, int reps, int level) {
+                float2* ck, const float* green, float norm, int reps, int level, int lo = 0, int hi = 0) {
   const int kx = level == 1 ? K_FFT_PM1 : level == 2 ? K_FFTX_PM2 : K_FFTX_PM3;
   const int ky = level == 1 ? K_FFT_PM1 : level == 2 ? K_FFTY_PM2 : K_FFTY_PM3;
   const int kz = level == 1 ? K_FFT_PM1 : level == 2 ? K_FFTZ_PM2 : K_FFTZ_PM3;
@@ -674,7 +678,7 @@ void launch_fft(cube_ctx* c, int n, int64_t nbox, const void* real_in, bool fixe
   // by n three times) as one multiplication by the reciprocal, rounded once from double
   const float inv = (float)(1.0 / std::pow((double)norm, (double)reps));
   if (c->fft_generic == 0 &&
-      fft2_dispatch(c, n, nbox, real_in, fixed, scale, phi_out, ck, green, inv, kx, ky, kz, kc, pt))
+      fft2_dispatch(c, n, nbox, real_in, fixed, scale, phi_out, ck, green, inv, kx, ky, kz, kc, pt, lo, hi > lo ? hi : n))
     return;
   const FFTDesc& D = *fft_desc(c, n);
   const int nh = n / 2 + 1;
@@ -1379,6 +1383,15 @@ static float dt_crit(float coef, float f2max, float a_mid) {
   return coef * std::sqrt(1.f / (std::sqrt(f2max) * a_mid * G_grid));
 }
 
+// The array cells in which a box's potential is read: its nfp physical cells and three around
+// them (the interpolation's outermost cell and its gradient); the whole mesh when a test
+// captures a potential of the level.
+static void phi_window(const cube_ctx* c, int level, int n, int nfp, int pad, int& lo, int& hi) {
+  const bool all = c->cap_level == level && c->cap_what == 1;
+  lo = all ? 0 : std::max(0, pad - 3);
+  hi = all ? n : std::min(n, pad + nfp + 3);
+}
+
 // ---- the kick in stages ----
 // PM1 and PM2, then the subtile classes.  Zeroes the kick's reductions first.
 static int enqueue_kick_a(cube_ctx* c) {
@@ -1446,8 +1459,10 @@ static int enqueue_kick_a(cube_ctx* c) {
         maybe_capture(c, 2, c->cap_box, 0, (char*)m.real + (c->cap_box - t0) * boxb, n, fixed, m.pt.rp, m.pt.psb);
       float* phi = reinterpret_cast<float*>(m.real);
       const float* k2 = kernel_table(c, 2, 0);
+      int w0, w1;
+      phi_window(c, 2, n, G.ngp, G.ngb, w0, w1);
       if (!k2) return CUBE_E_CUDA;
-      launch_fft(c, n, nb, m.real, fixed, G.mass_p, phi, m.ck, k2, (float)n * (float)n * (float)n, 1, 2);
+      launch_fft(c, n, nb, m.real, fixed, G.mass_p, phi, m.ck, k2, (float)n * (float)n * (float)n, 1, 2, w0, w1);
       if (c->cap_level == 2 && c->cap_box >= t0 && c->cap_box < t0 + nb)
         maybe_capture(c, 2, c->cap_box, 1, (char*)m.real + (c->cap_box - t0) * boxb, n, false, (int64_t)m.pt.pf * 4,
                       m.pt.psb);
@@ -1590,10 +1605,12 @@ static int enqueue_pm3(cube_ctx* c, const PM3Plan& pl, bool host_ires) {
         if (fixed) LAUNCH(c, K_DEP_PM3, 1, k_deposit_pm3<true><<<nblk(np), 256, 0, c->s>>>(G, np, c->xp, c->pcell, slots, cl, m.real, c->err, m.pt.pr, m.pt.plr));
         else LAUNCH(c, K_DEP_PM3, 1, k_deposit_pm3<false><<<nblk(np), 256, 0, c->s>>>(G, np, c->xp, c->pcell, slots, cl, m.real, c->err, m.pt.pr, m.pt.plr));
       }
+      int w0, w1;
+      phi_window(c, 3, n, G.nfp[cl], G.nfb[cl], w0, w1);
       const bool cap_here = cap_slot >= 0 && cap_chunk == k;
       if (cap_here) maybe_capture(c, 3, c->cap_box, 0, (char*)m.real + cap_slot * boxb, n, lint, m.pt.rp, m.pt.psb);
       float* phi = reinterpret_cast<float*>(m.real);
-      launch_fft(c, n, nb, m.real, lint, G.mass_p, phi, m.ck, g3, (float)n * (float)n * (float)n, 1, 3);
+      launch_fft(c, n, nb, m.real, lint, G.mass_p, phi, m.ck, g3, (float)n * (float)n * (float)n, 1, 3, w0, w1);
       if (cap_here)
         maybe_capture(c, 3, c->cap_box, 1, (char*)m.real + cap_slot * boxb, n, false, (int64_t)m.pt.pf * 4, m.pt.psb);
       const int nf = G.nfp[cl];

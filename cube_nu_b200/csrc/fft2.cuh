@@ -370,6 +370,8 @@ __global__ void __launch_bounds__(FcolBounds<N, TPS<R1, R2>::T>::MAXT, FcolBound
 // box.  One line per block, loaded when the block starts, two blocks per SM, left
 // the loads exposed: 4.63 ms for 512 boxes of 144^3, 3.1 ms now (1.9 at the copy bandwidth).
 // Column groups start at even columns, for the 16-byte copies; the row pitch is even.
+// Only planes [lo, hi) are written: the potential is read in the physical cells and three
+// cells around them, and the rest of the padding is not needed (k_fyx3_c2r).
 // ---------------------------------------------------------------------------------
 template <int N, int R1, int R2>
 struct ZLoop {
@@ -392,7 +394,7 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 template <int N, int R1, int R2>
 __global__ void __launch_bounds__(ZLoop<N, R1, R2>::THREADS, ZLoop<N, R1, R2>::MINB)
     k_fz_loop(float2* __restrict__ c, const float* __restrict__ green, const float2* __restrict__ gtw, int pc, int64_t plc,
-              int64_t nbox, int nsplit) {
+              int64_t nbox, int nsplit, int lo, int hi) {
   using Z = ZLoop<N, R1, R2>;
   constexpr int NH = Z::NH, WC = Z::WC, COLS = Z::COLS;
   extern __shared__ __align__(16) float2 sm[];
@@ -464,7 +466,10 @@ __global__ void __launch_bounds__(ZLoop<N, R1, R2>::THREADS, ZLoop<N, R1, R2>::M
       if (live) {
         float2* out = base(b) + col;
 #pragma unroll
-        for (int k2 = 0; k2 < R1; ++k2) out[(int64_t)(t + R2 * k2) * plc] = u[k2];
+        for (int k2 = 0; k2 < R1; ++k2) {
+          const int z = t + R2 * k2;
+          if (z >= lo && z < hi) out[(int64_t)z * plc] = u[k2];
+        }
       }
     }
   }
@@ -794,17 +799,19 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
   }
 }
 
+// Planes and rows [lo, hi) of each box (the part of the potential that is read; the whole box
+// with 0, N): at N = 48 that leaves out two fifths of the pass.
 template <int N, int R1, int R2>
 __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, R1, R2>::MINB) k_fyx3_c2r(const float2* __restrict__ c, float* __restrict__ r,
                                                                const float2* __restrict__ gtw, float inv,
-                                                               int pc, int pf, int64_t plc, int64_t plf) {
-  constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1, NP = N / 2;
+                                                               int pc, int pf, int64_t plc, int64_t plf, int lo, int hi) {
+  constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1;
   static_assert(T <= 16, "two sequences per warp");
   extern __shared__ float2 sm[];
   float2* tw = sm;
   float2* H = sm + N;  // half spectrum after the inverse y transforms, [N][NH]
   for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = gtw[i];
-  const int64_t plane = blockIdx.x;
+  const int64_t box = blockIdx.x / (unsigned)(hi - lo), plane = box * N + lo + (int)(blockIdx.x - box * (hi - lo));
   const float2* cp = c + plane * plc;
   float* rp = r + plane * plf;
   __syncthreads();
@@ -843,9 +850,10 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
     const int lane = threadIdx.x & 31, t = lane % L;
     const int g = (threadIdx.x >> 5) * (32 / L) + lane / L;
     constexpr int ngr = PlaneShape<N, R1, R2>::THREADS / L;
-    for (int p0 = 0; p0 < NP; p0 += ngr) {
+    const int p1 = (hi + 1) / 2;
+    for (int p0 = lo / 2; p0 < p1; p0 += ngr) {
       const int p = p0 + g;
-      const bool act = p < NP;
+      const bool act = p < p1;
       float2* H0 = H + (size_t)(act ? 2 * p : 0) * NH;  // rows 2p, 2p+1: 2*NH >= N contiguous slots
       const float2* H1 = H0 + NH;
       float2 v[R1];

@@ -62,6 +62,9 @@ __host__ __device__ inline int wrapi(int a, int n) {
   return a < 0 ? a + n : a;
 }
 
+// wrapi for a within one period of the range (-n <= a < 2n): no division.
+__host__ __device__ inline int wrap1(int a, int n) { return a < 0 ? a + n : a >= n ? a - n : a; }
+
 // Storage index of global coarse cell (gx,gy,gz) in the reference order
 // rhoc(nt,nt,nt,nnt,nnt,nnt): tile z,y,x outer, then cell z,y,x (x fastest).
 __host__ __device__ inline int64_t cell_index(const Geo& G, int gx, int gy, int gz) {

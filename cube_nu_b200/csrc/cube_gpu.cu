@@ -2903,8 +2903,9 @@ extern "C" int cube_gpu_power(cube_ctx* c, const cube_power_in* in, float* xi, i
   if (special) fft2_forward_dispatch(c, nw, mesh, pt, K_PK_FFT);
   else fft_forward_generic(c, nw, mesh, pt, K_PK_FFT);
   PK_CK(cudaMemsetAsync(bins, 0, nbins4 * sizeof(double), c->s));
-  smem_optin(k_pk_bin, nbins4 * sizeof(double));
-  LAUNCH(c, K_PK_BIN, 1, k_pk_bin<<<nred, 256, nbins4 * sizeof(double), c->s>>>(
+  const size_t smb = nbins4 * sizeof(double) + (size_t)nw * sizeof(float);
+  smem_optin(k_pk_bin, smb);
+  LAUNCH(c, K_PK_BIN, 1, k_pk_bin<<<nred, 256, smb, c->s>>>(
                              reinterpret_cast<const float2*>(mesh), nw, pt.pc, pt.plc, (int)nbin, (float)np, in->n_interp, bins));
   std::vector<double> hb(nbins4), hc(nbins3);
   int hmm[2];

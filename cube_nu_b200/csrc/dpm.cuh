@@ -35,9 +35,12 @@ __device__ __forceinline__ int dpm_w(float x, float w[3], float dw[3]) {
   return (int)fl;
 }
 
-__device__ __forceinline__ int dpm_wrap(int i, int n) {
-  i %= n;
-  return i < 0 ? i + n : i;
+// The mesh cells floor(x)-1 .. floor(x)+1 of a position, wrapped (one division).
+__device__ __forceinline__ void dpm_cells(int fl, int n, int c[3]) {
+  const int f = wrapi(fl, n);
+  c[0] = wrap1(f - 1, n);
+  c[1] = f;
+  c[2] = wrap1(f + 1, n);
 }
 
 // rho += m * W, into a mesh with row pitch pr and plane pitch pl (floats).
@@ -46,17 +49,17 @@ __global__ void k_dpm_deposit(int n, int64_t np, const float* __restrict__ x, fl
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np) return;
   float w[3][3], dw[3];
-  int f[3];
+  int f[3][3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) f[d] = dpm_w(x[3 * i + d], w[d], dw);
+  for (int d = 0; d < 3; ++d) dpm_cells(dpm_w(x[3 * i + d], w[d], dw), n, f[d]);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const int64_t z = (int64_t)dpm_wrap(f[2] - 1 + c, n) * pl;
+    const int64_t z = (int64_t)f[2][c] * pl;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      const int64_t y = (int64_t)dpm_wrap(f[1] - 1 + b, n) * pr;
+      const int64_t y = (int64_t)f[1][b] * pr;
 #pragma unroll
-      for (int a = 0; a < 3; ++a) atomicAdd(&rho[z + y + dpm_wrap(f[0] - 1 + a, n)], m * w[0][a] * w[1][b] * w[2][c]);
+      for (int a = 0; a < 3; ++a) atomicAdd(&rho[z + y + f[0][a]], m * w[0][a] * w[1][b] * w[2][c]);
     }
   }
 }
@@ -68,19 +71,19 @@ __global__ void k_dpm_kick(int n, int64_t np, const float* __restrict__ x, const
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np) return;
   float w[3][3], dw[3];
-  int f[3];
+  int f[3][3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) f[d] = dpm_w(x[3 * i + d], w[d], dw);
+  for (int d = 0; d < 3; ++d) dpm_cells(dpm_w(x[3 * i + d], w[d], dw), n, f[d]);
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const int64_t z = (int64_t)dpm_wrap(f[2] - 1 + c, n) * n * n;
+    const int64_t z = (int64_t)f[2][c] * n * n;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      const int64_t y = (int64_t)dpm_wrap(f[1] - 1 + b, n) * n;
+      const int64_t y = (int64_t)f[1][b] * n;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        const float4 F = __ldg(&fm[z + y + dpm_wrap(f[0] - 1 + a, n)]);
+        const float4 F = __ldg(&fm[z + y + f[0][a]]);
         const float ww = w[0][a] * w[1][b] * w[2][c];
         s0 += ww * F.x;
         s1 += ww * F.y;
@@ -104,29 +107,27 @@ __global__ void k_dpm_drift(int n, int64_t np3, float* __restrict__ x, const flo
   x[i] = y;
 }
 
-// lamF(c) += sum_i W(x_i - c) u_i (float4 mesh, dense, x fastest; .w unused).
+// lamF(c) += sum_i W(x_i - c) u_i (float4 mesh, dense, x fastest; .w unused).  One 16-byte
+// vector reduction per cell: three 4-byte ones took 0.74 ms for 128^3 particles.
 __global__ void k_dpm_deposit_vec(int n, int64_t np, const float* __restrict__ x, const float* __restrict__ u,
                                   float4* __restrict__ lam) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np) return;
   float w[3][3], dw[3];
-  int f[3];
+  int f[3][3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) f[d] = dpm_w(x[3 * i + d], w[d], dw);
+  for (int d = 0; d < 3; ++d) dpm_cells(dpm_w(x[3 * i + d], w[d], dw), n, f[d]);
   const float u0 = u[3 * i], u1 = u[3 * i + 1], u2 = u[3 * i + 2];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const int64_t z = (int64_t)dpm_wrap(f[2] - 1 + c, n) * n * n;
+    const int64_t z = (int64_t)f[2][c] * n * n;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      const int64_t y = (int64_t)dpm_wrap(f[1] - 1 + b, n) * n;
+      const int64_t y = (int64_t)f[1][b] * n;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        float* L = reinterpret_cast<float*>(&lam[z + y + dpm_wrap(f[0] - 1 + a, n)]);
         const float ww = w[0][a] * w[1][b] * w[2][c];
-        atomicAdd(L, ww * u0);
-        atomicAdd(L + 1, ww * u1);
-        atomicAdd(L + 2, ww * u2);
+        atomicAdd(&lam[z + y + f[0][a]], make_float4(ww * u0, ww * u1, ww * u2, 0.f));
       }
     }
   }
@@ -135,19 +136,19 @@ __global__ void k_dpm_deposit_vec(int n, int64_t np, const float* __restrict__ x
 // s(c) = (grad_h^T lamF)(c) = sum_d sum_o w_o lamF_d(c - o e_d), o in {-2,-1,1,2}, the
 // transpose of the 4-point gradient; written into a mesh with row pitch pr, plane pl.
 __global__ void k_dpm_grad_t(int n, const float4* __restrict__ lam, float* __restrict__ s, int pr, int64_t pl) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t n3 = (int64_t)n * n * n;
-  if (i >= n3) return;
-  const int x = (int)(i % n), y = (int)((i / n) % n), z = (int)(i / ((int64_t)n * n));
+  const unsigned un = (unsigned)n, i = blockIdx.x * blockDim.x + threadIdx.x;  // n < 1626
+  if (i >= un * un * un) return;
+  const unsigned zy = i / un;
+  const int x = (int)(i - zy * un), z = (int)(zy / un), y = (int)(zy - (unsigned)z * un);
   const float w[4] = {(CUBE_W_ALPHA - 1.f) / 4.f, -CUBE_W_ALPHA / 2.f, CUBE_W_ALPHA / 2.f, (1.f - CUBE_W_ALPHA) / 4.f};
   const int o[4] = {-2, -1, 1, 2};
   auto L = [&](int a, int b, int c) { return __ldg(&lam[((int64_t)c * n + b) * n + a]); };
   float t = 0.f;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    t += w[k] * L(dpm_wrap(x - o[k], n), y, z).x;
-    t += w[k] * L(x, dpm_wrap(y - o[k], n), z).y;
-    t += w[k] * L(x, y, dpm_wrap(z - o[k], n)).z;
+    t += w[k] * L(wrap1(x - o[k], n), y, z).x;
+    t += w[k] * L(x, wrap1(y - o[k], n), z).y;
+    t += w[k] * L(x, y, wrap1(z - o[k], n)).z;
   }
   s[(int64_t)z * pl + (int64_t)y * pr + x] = t;
 }
@@ -160,20 +161,20 @@ __global__ void k_dpm_grad_gather(int n, int64_t np, const float* __restrict__ x
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np) return;
   float w[3][3], dw[3][3];
-  int f[3];
+  int f[3][3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) f[d] = dpm_w(x[3 * i + d], w[d], dw[d]);
+  for (int d = 0; d < 3; ++d) dpm_cells(dpm_w(x[3 * i + d], w[d], dw[d]), n, f[d]);
   const float u0 = u ? u[3 * i] : 0.f, u1 = u ? u[3 * i + 1] : 0.f, u2 = u ? u[3 * i + 2] : 0.f;
   float g0 = 0.f, g1 = 0.f, g2 = 0.f;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const int zz = dpm_wrap(f[2] - 1 + c, n);
+    const int zz = f[2][c];
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      const int yy = dpm_wrap(f[1] - 1 + b, n);
+      const int yy = f[1][b];
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        const int xx = dpm_wrap(f[0] - 1 + a, n);
+        const int xx = f[0][a];
         float val = 0.f;
         if (u) {
           const float4 F = __ldg(&fm[((int64_t)zz * n + yy) * n + xx]);
@@ -189,16 +190,6 @@ __global__ void k_dpm_grad_gather(int n, int64_t np, const float* __restrict__ x
   gx[3 * i] += g0;
   gx[3 * i + 1] += g1;
   gx[3 * i + 2] += g2;
-}
-
-// Copy a pitched mesh (row pr, plane pl) into a dense n^3 array, or back.
-__global__ void k_dpm_copy(int n, const float* __restrict__ src, int spr, int64_t spl, float* __restrict__ dst, int dpr,
-                           int64_t dpl) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t n3 = (int64_t)n * n * n;
-  if (i >= n3) return;
-  const int x = (int)(i % n), y = (int)((i / n) % n), z = (int)(i / ((int64_t)n * n));
-  dst[(int64_t)z * dpl + (int64_t)y * dpr + x] = src[(int64_t)z * spl + (int64_t)y * spr + x];
 }
 
 }  // namespace cube

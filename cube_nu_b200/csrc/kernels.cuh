@@ -503,10 +503,10 @@ __global__ void __launch_bounds__(256) k_deposit_pm1(Geo G, int64_t np, const vo
   MassAcc<FIXED> mass;
 #pragma unroll
   for (int a3 = 0; a3 < 3; ++a3) {
-    const int64_t z = (int64_t)wrapi(g[2] - 1 + a3, nc) * pl;
+    const int64_t z = (int64_t)wrap1(g[2] - 1 + a3, nc) * pl;
 #pragma unroll
     for (int a2 = 0; a2 < 3; ++a2) {
-      const int64_t y = (int64_t)wrapi(g[1] - 1 + a2, nc) * pr;
+      const int64_t y = (int64_t)wrap1(g[1] - 1 + a2, nc) * pr;
 #pragma unroll
       for (int a1 = 0; a1 < 3; ++a1) {
         const float ww = __fmul_rn(__fmul_rn(w[0][a1], w[1][a2]), w[2][a3]);
@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(256) k_deposit_pm1(Geo G, int64_t np, const vo
           if (samebits & (1u << k)) q += o;
         }
         if (head) {
-          atomicAdd(mesh + z + y + wrapi(g[0] - 1 + a1, nc), q);
+          atomicAdd(mesh + z + y + wrap1(g[0] - 1 + a1, nc), q);
           if constexpr (FIXED) mass.v += q;
         }
       }
@@ -1489,16 +1489,19 @@ __global__ void k_interp_pm1(Geo G, int64_t np, const void* __restrict__ xp, con
 // (particle_mesh.f90:224-247): at every coarse cell j (0-based, periodic) the three
 // components grad4(phi(j-2), phi(j-1), phi(j+1), phi(j+2)), with the same FP32
 // operations as tsc_gather_force, stored as float4 (fx, fy, fz, 0), x fastest.
-__global__ void k_force_pm1(int nc, const float* __restrict__ phi, int pf, int64_t pl, float4* __restrict__ force) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t n3 = (int64_t)nc * nc * nc;
-  if (i >= n3) return;
-  const int x = (int)(i % nc), y = (int)((i / nc) % nc), z = (int)(i / ((int64_t)nc * nc));
+// Cell indices in 32 bits (contexts hold fewer than 2^32 cells) and wraps by comparison: with
+// 64-bit divisions it took 0.24 ms at 256^3, five times the write of the force mesh.
+__global__ void __launch_bounds__(256) k_force_pm1(int nc, const float* __restrict__ phi, int pf, int64_t pl,
+                                                   float4* __restrict__ force) {
+  const unsigned n = (unsigned)nc, i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= n * n * n) return;
+  const unsigned zy = i / n;
+  const int x = (int)(i - zy * n), z = (int)(zy / n), y = (int)(zy - (unsigned)z * n);
   const int64_t row = (int64_t)z * pl + (int64_t)y * pf, xl = (int64_t)z * pl + x;
   const float* ph = phi;
-  auto X = [&](int d) { return __ldg(&ph[row + wrapi(x + d, nc)]); };
-  auto Y = [&](int d) { return __ldg(&ph[xl + (int64_t)wrapi(y + d, nc) * pf]); };
-  auto Z = [&](int d) { return __ldg(&ph[(int64_t)wrapi(z + d, nc) * pl + (int64_t)y * pf + x]); };
+  auto X = [&](int d) { return __ldg(&ph[row + wrap1(x + d, nc)]); };
+  auto Y = [&](int d) { return __ldg(&ph[xl + (int64_t)wrap1(y + d, nc) * pf]); };
+  auto Z = [&](int d) { return __ldg(&ph[(int64_t)wrap1(z + d, nc) * pl + (int64_t)y * pf + x]); };
   force[i] = make_float4(grad4(X(-2), X(-1), X(1), X(2)), grad4(Y(-2), Y(-1), Y(1), Y(2)),
                          grad4(Z(-2), Z(-1), Z(1), Z(2)), 0.f);
 }
@@ -1526,9 +1529,9 @@ __global__ void k_interp_pm1_force(Geo G, int64_t np, const void* __restrict__ x
   int64_t jx[3], jy[3], jz[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    jx[a] = wrapi(i2[0] - 2 + a, nc);
-    jy[a] = (int64_t)wrapi(i2[1] - 2 + a, nc) * nc;
-    jz[a] = (int64_t)wrapi(i2[2] - 2 + a, nc) * nc * nc;
+    jx[a] = wrap1(i2[0] - 2 + a, nc);
+    jy[a] = (int64_t)wrap1(i2[1] - 2 + a, nc) * nc;
+    jz[a] = (int64_t)wrap1(i2[2] - 2 + a, nc) * nc * nc;
   }
   float sx = 0.f, sy = 0.f, sz = 0.f;
 #pragma unroll

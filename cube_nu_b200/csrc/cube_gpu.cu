@@ -448,24 +448,6 @@ MeshPtrs mesh_ptrs(cube_ctx* c, int n, int64_t, bool fixed) {
   return m;
 }
 
-// The owner-computes PM3 deposit covers a class when every region of DEP3_R x DEP3_R x
-// DEP3_RZ cells of its boxes draws on at most DEP3_MAXC coarse cells (same range as
-// dep3_krange).
-bool dep3_own_fits(const Geo& G, int iapm) {
-  const int nft = G.nft[iapm], nfb = G.nfb[iapm];
-  auto fdiv = [](int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); };
-  auto most = [&](int R) {
-    int mk = 0;
-    for (int o = 0; o < nft; o += R) {
-      const int e = std::min(R, nft - o);
-      const int klo = std::max(-1, fdiv(o - nfb - 2, nfb)), khi = std::min(G.ntt, fdiv(o + e - nfb + 1, nfb));
-      mk = std::max(mk, khi - klo + 1);
-    }
-    return (int64_t)mk;
-  };
-  return nfb > 0 && most(DEP3_R) * most(DEP3_R) * most(DEP3_RZ) <= DEP3_MAXC;
-}
-
 // How many boxes of side n fit in the arena.
 int64_t boxes_fit(cube_ctx* c, int n, bool fixed) {
   const size_t per = mesh_bytes(c, n, 1, fixed);
@@ -999,15 +981,15 @@ static int alloc_particles(cube_ctx* c, int64_t np) {
   // mesh arena: everything that fits of what the largest level needs, within 70% of free memory
   const Geo& G = c->G;
   const bool fixed = c->P.deposit_mode == CUBE_DEPOSIT_FIXED;
-  size_t need = std::max(mesh_bytes(c, G.nc, 1, fixed), mesh_bytes(c, G.ngt, c->ntiles, fixed));
-  need = std::max(need, mesh_bytes(c, G.nft[2], c->ns3, fixed));  // every subtile in the lightest class
+  size_t need = std::max(mesh_bytes(c, G.nc, 1, fixed), mesh_bytes(c, G.ngt, c->ntiles, false));
+  need = std::max(need, mesh_bytes(c, G.nft[2], c->ns3, false));  // every subtile in the lightest class
   for (int i = 3; i <= 5; ++i)
-    need = std::max(need, mesh_bytes(c, G.nft[i], std::max<int64_t>(1, c->ns3 / 16), fixed));
+    need = std::max(need, mesh_bytes(c, G.nft[i], std::max<int64_t>(1, c->ns3 / 16), false));
   size_t fre = 0, tot = 0;
   CK(cudaMemGetInfo(&fre, &tot));
   size_t budget = (size_t)(0.7 * (double)fre);
   size_t want = std::min(need, budget);
-  want = std::max(want, std::max(mesh_bytes(c, G.nc, 1, fixed), mesh_bytes(c, G.nft[5], 1, fixed)));
+  want = std::max(want, std::max(mesh_bytes(c, G.nc, 1, fixed), mesh_bytes(c, G.nft[5], 1, false)));
   if (c->arena) cudaFree(c->arena);
   c->arena = nullptr;
   CK(cudaMalloc(&c->arena, want));
@@ -1392,6 +1374,24 @@ static void phi_window(const cube_ctx* c, int level, int n, int nfp, int pad, in
   hi = all ? n : std::min(n, pad + nfp + 3);
 }
 
+static double per_cell(const cube_ctx* c) { return (double)c->np / (double)c->G.ncells; }
+
+// The PM2 or PM3 density of `nb` boxes into their float meshes (k_deposit_box); subs: the
+// boxes' subtiles, or null for tiles from t0.  msum: mass slots or null.
+static void enqueue_deposit(cube_ctx* c, int cls, const DepBox& B, int64_t nb, const int32_t* subs, int t0,
+                            const MeshPtrs& m, void* msum) {
+  const size_t sm = dep_box_smem(B);
+  const unsigned grid = (unsigned)(nb * B.ncx * B.ncy * B.ncz);
+  const bool fixed = c->P.deposit_mode == CUBE_DEPOSIT_FIXED;
+  auto run = [&](auto kernel, auto* codes) {
+    smem_optin(kernel, sm);
+    LAUNCH(c, cls, 1, kernel<<<grid, DEPB_T, sm, c->s>>>(c->G, B, codes, c->pcell, c->cstart, subs, t0,
+                                                         static_cast<float*>(m.real), m.pt.pr, m.pt.plr, fixed, msum));
+  };
+  if (c->G.izipx == 1) run(k_deposit_box<uint8_t>, static_cast<const uint8_t*>(c->xp));
+  else run(k_deposit_box<uint16_t>, static_cast<const uint16_t*>(c->xp));
+}
+
 // ---- the kick in stages ----
 // PM1 and PM2, then the subtile classes.  Zeroes the kick's reductions first.
 static int enqueue_kick_a(cube_ctx* c) {
@@ -1447,22 +1447,20 @@ static int enqueue_kick_a(cube_ctx* c) {
   // ---------------- PM2 (kick.f90:47-77) ----------------
   {
     const int n = G.ngt;
-    const int64_t per = std::min<int64_t>(G.tile1 - G.tile0, boxes_fit(c, n, fixed));
+    const int64_t per = std::min<int64_t>(G.tile1 - G.tile0, boxes_fit(c, n, false));
     for (int t0 = G.tile0; t0 < G.tile1; t0 += (int)per) {  // this rank's tiles
       const int nb = (int)std::min<int64_t>(per, G.tile1 - t0);
-      MeshPtrs m = mesh_ptrs(c, n, nb, fixed);
+      MeshPtrs m = mesh_ptrs(c, n, nb, false);
       const int64_t boxb = (int64_t)n * m.pt.psb;
-      CK(cudaMemsetAsync(m.real, 0, nb * boxb, c->s));
-      if (fixed) LAUNCH(c, K_DEP_PM2, 1, k_deposit_pm2<true><<<nblk(np), 256, 0, c->s>>>(G, np, c->xp, c->pcell, m.real, t0, nb, m.pt.pr, m.pt.plr, ms2));
-      else LAUNCH(c, K_DEP_PM2, 1, k_deposit_pm2<false><<<nblk(np), 256, 0, c->s>>>(G, np, c->xp, c->pcell, m.real, t0, nb, m.pt.pr, m.pt.plr, ms2));
+      enqueue_deposit(c, K_DEP_PM2, dep_box(G.nt, G.ncb, G.rcs, G.ngb, 0, nb, per_cell(c), c->nsm), nb, nullptr, t0, m, ms2);
       if (c->cap_level == 2 && c->cap_box >= t0 && c->cap_box < t0 + nb)
-        maybe_capture(c, 2, c->cap_box, 0, (char*)m.real + (c->cap_box - t0) * boxb, n, fixed, m.pt.rp, m.pt.psb);
+        maybe_capture(c, 2, c->cap_box, 0, (char*)m.real + (c->cap_box - t0) * boxb, n, false, m.pt.rp, m.pt.psb);
       float* phi = reinterpret_cast<float*>(m.real);
       const float* k2 = kernel_table(c, 2, 0);
       int w0, w1;
       phi_window(c, 2, n, G.ngp, G.ngb, w0, w1);
       if (!k2) return CUBE_E_CUDA;
-      launch_fft(c, n, nb, m.real, fixed, G.mass_p, phi, m.ck, k2, (float)n * (float)n * (float)n, 1, 2, w0, w1);
+      launch_fft(c, n, nb, m.real, false, G.mass_p, phi, m.ck, k2, (float)n * (float)n * (float)n, 1, 2, w0, w1);
       if (c->cap_level == 2 && c->cap_box >= t0 && c->cap_box < t0 + nb)
         maybe_capture(c, 2, c->cap_box, 1, (char*)m.real + (c->cap_box - t0) * boxb, n, false, (int64_t)m.pt.pf * 4,
                       m.pt.psb);
@@ -1500,7 +1498,6 @@ static int enqueue_kick_a(cube_ctx* c) {
 // of each class, the ones a captured step already covered.
 static PM3Plan make_plan(cube_ctx* c, const int32_t cnt[8], bool headroom, const int* skip = nullptr) {
   const Geo& G = c->G;
-  const bool fixed = c->P.deposit_mode == CUBE_DEPOSIT_FIXED;
   PM3Plan pl;
   memset(&pl, 0, sizeof(pl));
   int k = 0;
@@ -1515,8 +1512,7 @@ static PM3Plan make_plan(cube_ctx* c, const int32_t cnt[8], bool headroom, const
       pl.cap[cl] = 0;
       continue;
     }
-    const bool lint = fixed && !dep3_own_fits(G, cl);
-    const int64_t per = std::min<int64_t>(want, boxes_fit(c, G.nft[cl], lint));
+    const int64_t per = std::min<int64_t>(want, boxes_fit(c, G.nft[cl], false));
     pl.per[cl] = (int)per;
     pl.kbase[cl] = k;
     k += (int)((want + per - 1) / per);
@@ -1582,35 +1578,21 @@ static int enqueue_pm3(cube_ctx* c, const PM3Plan& pl, bool host_ires) {
     const int n = G.nft[cl];
     const float* g3 = kernel_table(c, 3, cl);
     if (!g3) return CUBE_E_CUDA;
-    const bool own = fixed && dep3_own_fits(G, cl);
-    const bool lint = fixed && !own;  // int64 mesh layout
     const int nch = (pl.cap[cl] + pl.per[cl] - 1) / pl.per[cl];
     for (int ch = 0; ch < nch; ++ch) {
       const int k = pl.kbase[cl] + ch;
       const int nb = std::min(pl.per[cl], pl.cap[cl] - ch * pl.per[cl]);
       const int32_t* slots = c->box_slot + (int64_t)k * c->ns3;
       const int32_t* subs = c->box_sub + (int64_t)k * pl.per_max;
-      MeshPtrs m = mesh_ptrs(c, n, nb, lint);
+      MeshPtrs m = mesh_ptrs(c, n, nb, false);
       const int64_t boxb = (int64_t)n * m.pt.psb;
-      if (own) {
-        // owner-computes deposit: writes every cell (as float), no memset
-        const int nr = (n + DEP3_R - 1) / DEP3_R, nrz = (n + DEP3_RZ - 1) / DEP3_RZ;
-        const size_t sm = (size_t)DEP3_R * DEP3_R * DEP3_RZ * 8;
-        smem_optin(k_deposit_pm3_own, sm);
-        LAUNCH(c, K_DEP_PM3, 1, k_deposit_pm3_own<<<(unsigned)((int64_t)nb * nr * nr * nrz), DEP3_THREADS, sm, c->s>>>(
-                                    G, c->xp, c->cstart, subs, cl, reinterpret_cast<float*>(m.real), c->err, m.pt.pr,
-                                    m.pt.plr, nr, nr, nrz));
-      } else {
-        CK(cudaMemsetAsync(m.real, 0, nb * boxb, c->s));
-        if (fixed) LAUNCH(c, K_DEP_PM3, 1, k_deposit_pm3<true><<<nblk(np), 256, 0, c->s>>>(G, np, c->xp, c->pcell, slots, cl, m.real, c->err, m.pt.pr, m.pt.plr));
-        else LAUNCH(c, K_DEP_PM3, 1, k_deposit_pm3<false><<<nblk(np), 256, 0, c->s>>>(G, np, c->xp, c->pcell, slots, cl, m.real, c->err, m.pt.pr, m.pt.plr));
-      }
+      enqueue_deposit(c, K_DEP_PM3, dep_box(G.ntt, 1, G.nfb[cl], G.nfb[cl], cl, nb, per_cell(c), c->nsm), nb, subs, 0, m, nullptr);
       int w0, w1;
       phi_window(c, 3, n, G.nfp[cl], G.nfb[cl], w0, w1);
       const bool cap_here = cap_slot >= 0 && cap_chunk == k;
-      if (cap_here) maybe_capture(c, 3, c->cap_box, 0, (char*)m.real + cap_slot * boxb, n, lint, m.pt.rp, m.pt.psb);
+      if (cap_here) maybe_capture(c, 3, c->cap_box, 0, (char*)m.real + cap_slot * boxb, n, false, m.pt.rp, m.pt.psb);
       float* phi = reinterpret_cast<float*>(m.real);
-      launch_fft(c, n, nb, m.real, lint, G.mass_p, phi, m.ck, g3, (float)n * (float)n * (float)n, 1, 3, w0, w1);
+      launch_fft(c, n, nb, m.real, false, G.mass_p, phi, m.ck, g3, (float)n * (float)n * (float)n, 1, 3, w0, w1);
       if (cap_here)
         maybe_capture(c, 3, c->cap_box, 1, (char*)m.real + cap_slot * boxb, n, false, (int64_t)m.pt.pf * 4, m.pt.psb);
       const int nf = G.nfp[cl];

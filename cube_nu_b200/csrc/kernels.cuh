@@ -411,15 +411,6 @@ __global__ void k_permute_ids(int64_t np, const uint32_t* __restrict__ ssrc, con
 // Deposit (particle_mesh.f90:20-109, kick.f90:611-691).
 // =================================================================================
 
-template <bool FIXED>
-__device__ __forceinline__ void dep_add(void* rho, int64_t i, float w) {
-  if (FIXED) {
-    atomicAdd(reinterpret_cast<unsigned long long*>(rho) + i, fixed40(w));
-  } else {
-    atomicAdd(reinterpret_cast<float*>(rho) + i, w);
-  }
-}
-
 // Mass sums of the deposited density over the physical cells of a level (the reference
 // forms them in real(8): particle_mesh.f90:106 testrho, kick.f90:687-688 ptotal), in
 // particle units.  The fixed-point form sums the int64 contributions exactly (order
@@ -534,84 +525,6 @@ __global__ void __launch_bounds__(256) k_deposit_pm1(Geo G, int64_t np, const vo
   mass.flush(msum);
 }
 
-// Candidate tiles along one dimension for a particle with global cell g: its own tile
-// and, within ncb of a tile face, the neighbour whose ghost region holds it.
-// Writes (tile, local coordinate i-1 in that tile) pairs; returns the count (1 or 2).
-__device__ __forceinline__ int tile_cands(const Geo& G, int g, int* t, int* li) {
-  const int tt = g / G.nt, l = g - tt * G.nt;
-  t[0] = tt;
-  li[0] = l;
-  // constant slot indices keep the caller's arrays in registers
-  const bool lo = l < G.ncb, hi = !lo && l >= G.nt - G.ncb;
-  t[1] = wrapi(lo ? tt - 1 : tt + 1, G.nnt);
-  li[1] = lo ? l + G.nt : l - G.nt;
-  return (lo || hi) ? 2 : 1;
-}
-
-// PM2 tile meshes [tile - tile0][ngt^3]; fine index i maps to array i-(1-ngb).
-template <bool FIXED>
-__global__ void __launch_bounds__(256, 5) k_deposit_pm2(Geo G, int64_t np, const void* __restrict__ xp, const int32_t* __restrict__ pcell,
-                              void* __restrict__ rho, int tile0, int ntile, int pr, int64_t pl, void* msum) {
-  const int64_t ip = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  MassAcc<FIXED> mass;
-  if (ip < np) {
-  int g[3];
-  cell_coords(G, pcell[ip], g[0], g[1], g[2]);
-  int tc[3][2], lc[3][2], nca[3];
-  double f[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    nca[d] = tile_cands(G, g[d], tc[d], lc[d]);
-    f[d] = zfrac(load_code(xp, G.izipx, 3 * ip + d), G);
-  }
-  const int ngt = G.ngt;
-  const int64_t box = (int64_t)ngt * pl;  // elements per box
-  // Candidate loops fully unrolled (at most two per dimension) so the candidate arrays
-  // stay in registers.
-#pragma unroll
-  for (int cz = 0; cz < 2; ++cz)
-#pragma unroll
-    for (int cy = 0; cy < 2; ++cy)
-#pragma unroll
-      for (int cx = 0; cx < 2; ++cx) {
-        if (cz >= nca[2] || cy >= nca[1] || cx >= nca[0]) continue;
-        const int T = (tc[2][cz] * G.nnt + tc[1][cy]) * G.nnt + tc[0][cx];
-        if (T < tile0 || T >= tile0 + ntile) continue;
-        const int l[3] = {lc[0][cx], lc[1][cy], lc[2][cz]};
-        int i2[3];
-        float w[3][3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const double xpos = ((double)l[d] + f[d]) * (double)G.rcs;  // /gridsize(=1)
-          i2[d] = tsc_weights(xpos, w[d]);
-        }
-        char* base = (char*)rho + (int64_t)(T - tile0) * box * (FIXED ? 8 : 4);
-#pragma unroll
-        for (int a3 = 0; a3 < 3; ++a3) {
-          const int z = i2[2] - 1 + a3 - (1 - G.ngb);
-          if (z < 0 || z >= ngt) continue;
-#pragma unroll
-          for (int a2 = 0; a2 < 3; ++a2) {
-            const int y = i2[1] - 1 + a2 - (1 - G.ngb);
-            if (y < 0 || y >= ngt) continue;
-#pragma unroll
-            for (int a1 = 0; a1 < 3; ++a1) {
-              const int x = i2[0] - 1 + a1 - (1 - G.ngb);
-              if (x < 0 || x >= ngt) continue;
-              const float ww = __fmul_rn(__fmul_rn(w[0][a1], w[1][a2]), w[2][a3]);
-              dep_add<FIXED>(base, (int64_t)z * pl + (int64_t)y * pr + x, ww);
-              // physical cells 1..ngp of the tile (array ngb..ngb+ngp-1)
-              if ((unsigned)(x - G.ngb) < (unsigned)G.ngp && (unsigned)(y - G.ngb) < (unsigned)G.ngp &&
-                  (unsigned)(z - G.ngb) < (unsigned)G.ngp)
-                mass.add(ww);
-            }
-          }
-        }
-      }
-  }
-  mass.flush(msum);
-}
-
 // Candidate subtiles along one dimension (PM3 nloop=1): own subtile and, in the
 // first/last coarse cell of a subtile, the neighbour subtile (possibly in the
 // neighbour tile).  Returns count; writes tile, subtile, and local coordinate (i-1)
@@ -652,72 +565,6 @@ __device__ __forceinline__ int subtile_id(const Geo& G, const int t[3], const in
 __device__ __forceinline__ double pm3_xpos(double lf, const Geo& G, double gs, int rsf, int unfp) {
   const double a = lf * (double)G.rcs;
   return (((rsf & (rsf - 1)) == 0) ? a * (double)rsf : a / gs) - (double)unfp;
-}
-
-template <bool FIXED>
-__global__ void k_deposit_pm3(Geo G, int64_t np, const void* __restrict__ xp, const int32_t* __restrict__ pcell,
-                              const int32_t* __restrict__ box_slot, int iapm, void* __restrict__ rho,
-                              unsigned* err, int pr, int64_t pl) {
-  const int64_t ip = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (ip >= np) return;
-  int g[3];
-  cell_coords(G, pcell[ip], g[0], g[1], g[2]);
-  int tc[3][2], uc[3][2], lc[3][2], nca[3];  // at most two candidate subtiles per dimension (ntt >= 2)
-  double f[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    nca[d] = sub_cands(G, g[d], tc[d], uc[d], lc[d]);
-    f[d] = zfrac(load_code(xp, G.izipx, 3 * ip + d), G);
-  }
-  const int nft = G.nft[iapm], nfp = G.nfp[iapm], nfb = G.nfb[iapm];
-  const int64_t box = (int64_t)nft * pl;  // elements per box
-  const double gs = (double)(1.f / (float)rsf_of(iapm));  // pm%gridsize, real4
-  // Candidate loops fully unrolled (at most two per dimension) so the candidate arrays
-  // stay in registers.
-#pragma unroll
-  for (int cz = 0; cz < 2; ++cz)
-#pragma unroll
-    for (int cy = 0; cy < 2; ++cy)
-#pragma unroll
-      for (int cx = 0; cx < 2; ++cx) {
-        if (cz >= nca[2] || cy >= nca[1] || cx >= nca[0]) continue;
-        const int t[3] = {tc[0][cx], tc[1][cy], tc[2][cz]};
-        const int u[3] = {uc[0][cx], uc[1][cy], uc[2][cz]};
-        const int slot = box_slot[subtile_id(G, t, u)];
-        if (slot < 0) continue;
-        const int l[3] = {lc[0][cx], lc[1][cy], lc[2][cz]};
-        int i2[3];
-        float w[3][3];
-        bool oob = false;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const double xpos = pm3_xpos((double)l[d] + f[d], G, gs, rsf_of(iapm), u[d] * nfp);  // kick.f90:628-629
-          i2[d] = tsc_weights(xpos, w[d]);
-          if (i2[d] - 1 < -nfb || i2[d] + 1 > nfp + nfb + 1) oob = true;
-        }
-        if (oob) {
-          set_err(err, CUBE_DEVERR_DEPOSIT_RANGE);
-          continue;
-        }
-        char* base = (char*)rho + (int64_t)slot * box * (FIXED ? 8 : 4);
-#pragma unroll
-        for (int a3 = 0; a3 < 3; ++a3) {
-          const int z = i2[2] - 1 + a3 - (1 - nfb);
-          if (z < 0 || z >= nft) continue;
-#pragma unroll
-          for (int a2 = 0; a2 < 3; ++a2) {
-            const int y = i2[1] - 1 + a2 - (1 - nfb);
-            if (y < 0 || y >= nft) continue;
-#pragma unroll
-            for (int a1 = 0; a1 < 3; ++a1) {
-              const int x = i2[0] - 1 + a1 - (1 - nfb);
-              if (x < 0 || x >= nft) continue;
-              const float ww = __fmul_rn(__fmul_rn(w[0][a1], w[1][a2]), w[2][a3]);
-              dep_add<FIXED>(base, (int64_t)z * pl + (int64_t)y * pr + x, ww);
-            }
-          }
-        }
-      }
 }
 
 // PM3 mass over the physical cells of every subtile box (kick.f90:687-688 ptotal), summed
@@ -887,209 +734,329 @@ __global__ void __launch_bounds__(MASS3_T) k_mass_pm3(Geo G, const int64_t* __re
 // thread) where most blocks only look.
 inline int mass3_groups(int64_t ncells) { return ncells <= (1 << 18) ? 1 : MASS3_T / 32; }
 
-// Owner-computes form of the fixed-point PM3 deposit: one block per region of
-// DEP3_R x DEP3_R x DEP3_RZ cells of one box.  The block sums, in shared memory, the contributions of the
-// particles of every coarse cell whose TSC footprint can reach the region, then writes
-// every cell of the region (zeros included) with plain stores, so the mesh needs no
-// memset and no cell is read back from DRAM.  Cells are written as the float the forward
-// FFT would convert the int64 sum to, (float)(q * 2^-40) (unscaled; the FFT multiplies by
-// the particle mass), into the float mesh layout: half the bytes of the int64 mesh, and
-// the FFT input is bit-identical.  Particle arithmetic is that of
-// k_deposit_pm3 (a box's candidate particles are those of coarse cells k = -1..ntt
-// around its subtile, with tile-local coordinate l = u*ntt + k), so the int64 sums are
-// identical.  Requires at most DEP3_MAXC candidate coarse cells per region (checked on
-// the host); the padding of the float layouts is left alone (the FFT never reads it).
-constexpr int DEP3_R = 24;   // region extent in x and y (cells)
-constexpr int DEP3_RZ = 24;  // region extent in z
-constexpr int DEP3_MAXC = 125;
-constexpr int DEP3_THREADS = 512;
-constexpr int DEP3_MINB = 2;  // blocks per SM
-constexpr int DEP3_SPLIT_MAX = 4095;
+// =================================================================================
+// PM2 and PM3 deposit, owner-computes, both deposit forms.  A box (a PM2 tile or a PM3
+// subtile) is S coarse cells a side and a halo of `halo`, q mesh cells a coarse cell, and its
+// mesh is padded by `pad` cells (halo*q, unless ngb says otherwise): the particles of coarse
+// cell k (relative to the box, -halo .. S+halo-1) lie in array cells k*q+pad .. +q-1 and reach
+// one cell further.  A block owns a column of cx x cy cells of a
+// box and planes [p0, p1) of it, and walks the coarse layers along z once: the contributions
+// of a layer's particles are summed in shared memory, in a ring of the q+2 planes a layer
+// reaches, and the planes no later layer reaches are written out (zeros included) and their
+// slots cleared.  So a particle is looked at by the columns it touches only (1.4 to 2.5 times
+// as a whole), the mesh needs no memset, and nothing is read back.
+//
+// Sums are int64 in units of 2^-40, round(w * 2^40) per contribution, so they are exact and
+// independent of the order; cells are written as the float they round to (unscaled; the FFT
+// multiplies by the particle mass).  Where no coarse cell the part reads holds more than
+// DEPB_CELL particles, a contribution is added as two independent 32-bit halves, a multiple
+// of 2^20 and a signed remainder, made by adding and subtracting 1.5 * 2^23 (round to
+// nearest) instead of a 64-bit conversion.  Else the low word is added first and its carry
+// goes into the high word: the 64-bit shared-memory atomic is a loop of compare-and-swap,
+// which made tiles with 64 particles a cell take 2.5 times as long.
+//
+// The halves lie in arrays of their own, so that a warp's additions fall on all 32 banks and
+// the write-out reads and clears them without conflicts (side by side, bank conflicts took
+// half of the shared-memory pipe's time, which was 72% busy).  One region of 24^3 cells per block, which looked at 4.6 times
+// its particles and took the whole 27-cell loop in nearly every warp, took 4.64 ms for 512
+// boxes of 144^3 and the PM2 reductions into memory 2.19 ms for eight of 288^3.
+// =================================================================================
+constexpr int DEPB_T = 320, DEPB_SEG = 96;
+constexpr int DEPB_SMEM = 96 * 1024;  // ring of one block: two blocks per SM
+// A cell takes contributions from 2^3 coarse cells (3^3 when a mesh cell is as large as one):
+// with at most 4095 of them, remainders of at most 2^19 stay below 2^31.
+constexpr int DEPB_CELL = 511, DEPB_CELL_Q1 = 151;
+
+struct DepBox {
+  int S, halo, q, pad, n;        // coarse cells, halo, mesh cells per coarse cell, padding and side of the mesh
+  int iapm;                      // PM3 class, 0 for PM2
+  int cx, cy, cz, ncx, ncy, ncz;  // cells of a block's part and the parts per dimension
+};
 
 __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
-// Candidate coarse-cell range (box-relative k) along one dimension for region cells
-// [o, o+e): TSC footprints fl+nfb-1..fl+nfb+1, one cell of margin for the FP64 rounding
-// of xpos.
-__device__ __forceinline__ void dep3_krange(int o, int e, int nfb, int ntt, int& klo, int& nk) {
-  klo = max(-1, floor_div(o - nfb - 2, nfb));
-  const int khi = min(ntt, floor_div(o + e - nfb + 1, nfb));
-  nk = khi - klo + 1;
-}
-
-__global__ void __launch_bounds__(DEP3_THREADS, DEP3_MINB) k_deposit_pm3_own(Geo G, const void* __restrict__ xp,
-                                                                     const int64_t* __restrict__ cstart,
-                                                                     const int32_t* __restrict__ box_sub, int iapm,
-                                                                     float* __restrict__ rho, unsigned* err,
-                                                                     int pr, int64_t pl, int nrx, int nry, int nrz) {
-  constexpr int R = DEP3_R, RZ = DEP3_RZ;
-  static_assert(R % 2 == 0 && R / 2 <= 16, "a half warp writes one region row");
-  extern __shared__ __align__(16) unsigned long long acc[];  // [RZ][R][R]
-  __shared__ int64_t cst[DEP3_MAXC];
-  __shared__ int ccnt[DEP3_MAXC], ckk[DEP3_MAXC], cpre[DEP3_MAXC + 1];
+template <typename CODE>
+__global__ void __launch_bounds__(DEPB_T, 2) k_deposit_box(Geo G, DepBox B, const CODE* __restrict__ xp,
+                                                           const int32_t* __restrict__ pcell,
+                                                           const int64_t* __restrict__ cstart,
+                                                           const int32_t* __restrict__ box_sub, int box0,
+                                                           float* __restrict__ rho, int pr, int64_t pl, bool fixed,
+                                                           void* msum) {
+  extern __shared__ __align__(16) int ring[];  // low words [q+2][cy][cx], then the high words
+  __shared__ int64_t seg_ip[2][DEPB_SEG];                     // a segment's first particle,
+  __shared__ int32_t seg_cell[2][DEPB_SEG], seg_k[2][DEPB_SEG], seg_pre[2][DEPB_SEG + 1];  // first cell, its k, prefix
+  __shared__ int dense;
   const int tid = threadIdx.x;
-  const int nft = G.nft[iapm], nfp = G.nfp[iapm], nfb = G.nfb[iapm];
-  const int nreg = nrx * nry * nrz;
-  const int64_t j = blockIdx.x / nreg;
-  const int r = (int)(blockIdx.x - j * nreg);
-  const int o[3] = {(r % nrx) * R, ((r / nrx) % nry) * R, (r / (nrx * nry)) * RZ};
-  const int e[3] = {min(R, nft - o[0]), min(R, nft - o[1]), min(RZ, nft - o[2])};
-  // subtile of this box; -1 pads a class list beyond its count (the slot is never read)
-  const int s = box_sub[j];
-  if (s < 0) return;
-  const int nns3 = G.nns * G.nns * G.nns;
-  const int T = s / nns3, f = s - T * nns3;
-  const int t[3] = {T % G.nnt, (T / G.nnt) % G.nnt, T / (G.nnt * G.nnt)};
-  const int u[3] = {f % G.nns, (f / G.nns) % G.nns, f / (G.nns * G.nns)};
-  int klo[3], nk[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) dep3_krange(o[d], e[d], nfb, G.ntt, klo[d], nk[d]);
-  const int ncand = nk[0] * nk[1] * nk[2];
-  if (ncand > DEP3_MAXC) {  // block-uniform; the host sizes regions so this does not happen
-    if (tid == 0) set_err(err, CUBE_DEVERR_DEPOSIT_RANGE);
-    return;
+  const int nparts = B.ncx * B.ncy * B.ncz;
+  const int64_t j = blockIdx.x / nparts;
+  const int part = (int)(blockIdx.x - j * nparts);
+  // origin of the box in coarse cells
+  int org[3], u[3] = {0, 0, 0};
+  if (box_sub) {  // a class list of subtiles; -1 pads it beyond its count (the slot is never read)
+    const int s = box_sub[j];
+    if (s < 0) return;
+    const int nns3 = G.nns * G.nns * G.nns, T = s / nns3, f = s - T * nns3;
+    u[0] = f % G.nns;
+    u[1] = (f / G.nns) % G.nns;
+    u[2] = f / (G.nns * G.nns);
+    org[0] = (T % G.nnt) * G.nt + u[0] * G.ntt;
+    org[1] = ((T / G.nnt) % G.nnt) * G.nt + u[1] * G.ntt;
+    org[2] = (T / (G.nnt * G.nnt)) * G.nt + u[2] * G.ntt;
+  } else {
+    const int T = box0 + (int)j;
+    org[0] = (T % G.nnt) * G.nt;
+    org[1] = ((T / G.nnt) % G.nnt) * G.nt;
+    org[2] = (T / (G.nnt * G.nnt)) * G.nt;
   }
-  // one thread per candidate coarse cell: its particle range and box-relative k
-  if (tid < ncand) {
-    const int kx = klo[0] + tid % nk[0], ky = klo[1] + (tid / nk[0]) % nk[1], kz = klo[2] + tid / (nk[0] * nk[1]);
-    const int64_t cell = cell_index(G, t[0] * G.nt + u[0] * G.ntt + kx, t[1] * G.nt + u[1] * G.ntt + ky,
-                                    t[2] * G.nt + u[2] * G.ntt + kz);
-    const int64_t a = cstart[cell];
-    cst[tid] = a;
-    ccnt[tid] = (int)(cstart[cell + 1] - a);
-    ckk[tid] = (kx + 1) | ((ky + 1) << 10) | ((kz + 1) << 20);
-  }
-  {
-    ulonglong2* a2 = reinterpret_cast<ulonglong2*>(acc);
-    for (int i = tid; i < R * R * RZ / 2; i += blockDim.x) a2[i] = make_ulonglong2(0ull, 0ull);
-  }
-  __syncthreads();
-  if (tid < 32) {  // prefix of the counts
+  const int q = B.q, rd = q + 2, cx = B.cx, cy = B.cy;
+  const int hi_at = rd * cy * cx;  // offset of the high words (a multiple of 4)
+  const int ox = (part % B.ncx) * cx, oy = ((part / B.ncx) % B.ncy) * cy, p0 = (part / (B.ncx * B.ncy)) * B.cz;
+  const int ex = min(cx, B.n - ox), ey = min(cy, B.n - oy), p1 = min(B.n, p0 + B.cz);
+  // coarse cells l = k + halo whose particles can reach the part: cells l*q+off-1 .. l*q+off+q
+  const int off = B.pad - B.halo * q, nl = B.S + 2 * B.halo;
+  const int kx0 = max(0, floor_div(ox - off - 1, q)) - B.halo, kx1 = min(nl - 1, floor_div(ox + ex - off, q)) - B.halo;
+  const int ky0 = max(0, floor_div(oy - off - 1, q)) - B.halo, ky1 = min(nl - 1, floor_div(oy + ey - off, q)) - B.halo;
+  const int l0 = min(nl - 1, max(0, floor_div(p0 - off - 1, q))), l1 = max(l0, min(nl - 1, floor_div(p1 - off, q)));
+  const int nseg = 3 * max(0, ky1 - ky0 + 1);  // per layer: rows of cells, cut where they leave the box's own cells
+  auto segment = [&](int i, int l, int& cell, int& kx) {  // first cell and k of segment i; returns its cells
+    const int row = i / 3, piece = i - 3 * row;
+    const int lo = piece == 0 ? kx0 : piece == 1 ? max(kx0, 0) : max(kx0, B.S);
+    const int hi = piece == 0 ? min(kx1, -1) : piece == 1 ? min(kx1, B.S - 1) : kx1;
+    kx = lo;
+    if (lo > hi) return 0;
+    cell = (int)cell_index(G, org[0] + lo, org[1] + ky0 + row, org[2] + l - B.halo);
+    return hi - lo + 1;
+  };
+  auto table = [&](int buf, int l) {  // one warp: the segments of layer l
+    const int lane = tid & 31;
     int carry = 0;
-    for (int b0 = 0; b0 < ncand; b0 += 32) {
-      const int i = b0 + tid;
-      int incl = (i < ncand) ? ccnt[i] : 0;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, off);
-        if (tid >= off) incl += v;
+    for (int i0 = 0; i0 < nseg; i0 += 32) {
+      const int i = i0 + lane;
+      int cell = 0, kx = 0, cnt = 0;
+      int64_t ip = 0;
+      if (i < nseg) {
+        const int m = segment(i, l, cell, kx);
+        if (m) {
+          ip = cstart[cell];
+          cnt = (int)(cstart[cell + m] - ip);
+        }
       }
-      if (i < ncand) cpre[i + 1] = carry + incl;
+      int incl = cnt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (i < nseg) {
+        seg_ip[buf][i] = ip;
+        seg_cell[buf][i] = cell;
+        seg_k[buf][i] = (kx + B.halo) | ((i / 3 + ky0 + B.halo) << 16);
+        seg_pre[buf][i + 1] = carry + incl;
+      }
       carry += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (tid == 0) cpre[0] = 0;
+    if (lane == 0) seg_pre[buf][0] = 0;
+  };
+  if (tid == 0) dense = 0;
+  {
+    int4* z = reinterpret_cast<int4*>(ring);
+    for (int i = tid; i < rd * cy * cx / 2; i += DEPB_T) z[i] = make_int4(0, 0, 0, 0);
   }
   __syncthreads();
-  const int total = cpre[ncand];
-  const int rsf = rsf_of(iapm);
-  const double gs = (double)(1.f / (float)rsf);  // pm%gridsize, real4
-  // Each q = round(w * 2^40) <= 2^40.  With at most DEP3_SPLIT_MAX candidate particles no
-  // cell takes more than that many contributions, so the low 20 bits and the rest of q
-  // can be summed in the two 32-bit halves of the cell without overflow:
-  // sum q = (sum hi << 20) + sum lo.  Denser regions use 64-bit atomics.
-  const bool split = total <= DEP3_SPLIT_MAX;
-  // the visit loop, instantiated for each summation form (block-uniform choice)
-  auto visits = [&](auto split_tag) {
-    constexpr bool SPLIT = decltype(split_tag)::value;
-    for (int v = tid; v < total; v += blockDim.x) {
-      int lo = 0, hi = ncand;
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (cpre[mid] <= v) lo = mid;
-        else hi = mid;
-      }
-      const int64_t ip = cst[lo] + (v - cpre[lo]);
-      const int kk = ckk[lo];
-      const int k[3] = {(kk & 1023) - 1, ((kk >> 10) & 1023) - 1, (kk >> 20) - 1};
-      int code[3];
+  for (int i = tid; i < (l1 - l0 + 1) * nseg; i += DEPB_T) {
+    const int l = i / nseg;
+    int cell, kx;
+    const int m = segment(i - l * nseg, l0 + l, cell, kx);
+    for (int k = 0; k < m; ++k)
+      if (cstart[cell + k + 1] - cstart[cell + k] > (q > 1 ? DEPB_CELL : DEPB_CELL_Q1)) dense = 1;
+  }
+  if (tid < 32) table(0, l0);
+  __syncthreads();
+  const bool split = dense == 0;
+  const bool pow2 = (q & (q - 1)) == 0;
+  const int rsf = B.iapm ? rsf_of(B.iapm) : 1;
+  const double gs = (double)(1.f / (float)rsf);
+  const int bits = 8 * (int)sizeof(CODE);
+  const float M = 12582912.f;  // 1.5 * 2^23
+  // write-out: a thread's 4 cells of a plane, planes dealt to groups of threads
+  const int cxq = cx / 4, per = cxq * cy, ngrp = max(1, DEPB_T / per), gstep = ngrp % rd;
+  int done = p0;  // planes written
+  unsigned long long mloc = 0;
+  for (int l = l0; l <= l1; ++l) {
+    const int buf = (l - l0) & 1;
+    if (tid < 32 && l < l1) table(buf ^ 1, l + 1);
+    const int total = seg_pre[buf][nseg];
+    const int zb = l * q + off - 1;  // first plane the layer reaches; the last is zb + q + 1
+    const int zslot = (zb % rd + rd) % rd;
+    auto visits = [&](auto split_tag) {
+      constexpr bool SPLIT = decltype(split_tag)::value;
+      for (int v = tid; v < total; v += DEPB_T) {
+        int lo = 0, hi = nseg;
+        while (hi - lo > 1) {
+          const int mid = (lo + hi) >> 1;
+          if (seg_pre[buf][mid] <= v) lo = mid;
+          else hi = mid;
+        }
+        const int64_t ip = seg_ip[buf][lo] + (v - seg_pre[buf][lo]);
+        const int kk = seg_k[buf][lo];
+        const int k[3] = {(kk & 0xffff) + (pcell[ip] - seg_cell[buf][lo]), kk >> 16, l};  // k + halo
+        int c0[3];  // part-local cell of the footprint's first weight
+        float w[3][3];
+        const int o[3] = {ox, oy, zb};
 #pragma unroll
-      for (int d = 0; d < 3; ++d) code[d] = load_code(xp, G.izipx, 3 * ip + d);
-      int i2[3], c0[3];
-      float w[3][3];
-      bool oob = false, miss = false;
+        for (int d = 0; d < 3; ++d) {
+          const unsigned code = (unsigned)xp[3 * ip + d];
+          if (pow2) {
+            // (code + 1/2) q / 2^bits: whole part and, exactly, the rest
+            const unsigned t = (2u * code + 1u) * (unsigned)q;
+            const float f = (float)(t & ((2u << bits) - 1u)) * (0.5f / (float)(1u << bits));
+            const float a = __fsub_rn(1.f, f);
+            w[d][0] = __fmul_rn(__fmul_rn(a, a), 0.5f);
+            w[d][2] = __fmul_rn(__fmul_rn(f, f), 0.5f);
+            w[d][1] = __fsub_rn(__fsub_rn(1.f, w[d][0]), w[d][2]);
+            c0[d] = k[d] * q + off + (int)(t >> (bits + 1)) - 1 - o[d];
+          } else {
+            const int nfp = B.S * q;
+            const double xpos = pm3_xpos((double)(u[d] * G.ntt + k[d] - B.halo) + zfrac((int)code, G), G, gs, rsf, u[d] * nfp);
+            c0[d] = tsc_weights(xpos, w[d]) + B.pad - 2 - o[d];  // kick.f90:628-629
+          }
+        }
+        if (c0[0] + 2 < 0 || c0[0] >= ex || c0[1] + 2 < 0 || c0[1] >= ey) continue;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const double xpos = pm3_xpos((double)(u[d] * G.ntt + k[d]) + zfrac(code[d], G), G, gs, rsf, u[d] * nfp);
-        i2[d] = tsc_weights(xpos, w[d]);  // kick.f90:628-629
-        if (i2[d] - 1 < -nfb || i2[d] + 1 > nfp + nfb + 1) oob = true;
-        c0[d] = i2[d] + nfb - 2 - o[d];  // region-local cell of the footprint's first weight
-        if (c0[d] + 2 < 0 || c0[d] >= e[d]) miss = true;
-      }
-      if (oob) {
-        set_err(err, CUBE_DEVERR_DEPOSIT_RANGE);
-        continue;
-      }
-      if (miss) continue;
+        for (int a3 = 0; a3 < 3; ++a3) {
+          const int zr = c0[2] + a3;  // 0 .. q+1: plane zb + zr
+          if (zb + zr < p0 || zb + zr >= p1) continue;
+          int slot = zslot + zr;
+          slot = slot >= rd ? slot - rd : slot;
+          // a power of two commutes with the products' rounding
+          const float wz = SPLIT ? __fmul_rn(w[2][a3], 1048576.f) : w[2][a3];
 #pragma unroll
-      for (int a3 = 0; a3 < 3; ++a3) {
-        const int z = c0[2] + a3;
-        if (z < 0 || z >= e[2]) continue;
+          for (int a2 = 0; a2 < 3; ++a2) {
+            const int y = c0[1] + a2;
+            if ((unsigned)y >= (unsigned)ey) continue;
+            int* const row = ring + (slot * cy + y) * cx + c0[0];
 #pragma unroll
-        for (int a2 = 0; a2 < 3; ++a2) {
-          const int y = c0[1] + a2;
-          if (y < 0 || y >= e[1]) continue;
-#pragma unroll
-          for (int a1 = 0; a1 < 3; ++a1) {
-            const int x = c0[0] + a1;
-            if (x < 0 || x >= e[0]) continue;
-            const float ww = __fmul_rn(__fmul_rn(w[0][a1], w[1][a2]), w[2][a3]);
-            const unsigned long long q = fixed40(ww);
-            unsigned long long* cell = &acc[(z * R + y) * R + x];
-            if (SPLIT) {
-              unsigned* h = reinterpret_cast<unsigned*>(cell);
-              atomicAdd(h, (unsigned)(q & 0xfffffull));
-              atomicAdd(h + 1, (unsigned)(q >> 20));
-            } else {
-              atomicAdd(cell, q);
+            for (int a1 = 0; a1 < 3; ++a1) {
+              if ((unsigned)(c0[0] + a1) >= (unsigned)ex) continue;
+              const float ww = __fmul_rn(__fmul_rn(w[0][a1], w[1][a2]), wz);
+              if (SPLIT) {
+                const float h = __fadd_rn(ww, M);
+                const float r = __fmaf_rn(__fsub_rn(ww, __fsub_rn(h, M)), 1048576.f, M);
+                atomicAdd(row + a1, __float_as_int(r) - __float_as_int(M));
+                atomicAdd(row + hi_at + a1, __float_as_int(h) - __float_as_int(M));
+              } else {
+                const unsigned long long v64 = fixed40(ww);
+                unsigned* const word = reinterpret_cast<unsigned*>(row + a1);
+                const unsigned old = atomicAdd(word, (unsigned)v64);
+                const unsigned up = (unsigned)(v64 >> 32) + (old + (unsigned)v64 < old ? 1u : 0u);
+                if (up) atomicAdd(word + hi_at, up);
+              }
             }
           }
         }
       }
+    };
+    if (split) visits(std::true_type{});
+    else visits(std::false_type{});
+    __syncthreads();
+    const int upto = l == l1 ? p1 : min(p1, zb + q);
+    for (int t = tid; t < per * ngrp; t += DEPB_T) {
+      const int grp = t / per, i = t - grp * per, y = i / cxq, x = 4 * (i - y * cxq);
+      if (y >= ey) continue;
+      int p = done + grp, slot = p % rd;
+      float* out = rho + (j * B.n + p) * pl + (int64_t)(oy + y) * pr + ox + x;
+      const bool vec = x + 4 <= ex && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && (pl & 3) == 0;
+      for (; p < upto; p += ngrp, out += ngrp * pl) {
+        float f[4] = {0.f, 0.f, 0.f, 0.f};
+        if (p >= zb && p <= zb + q + 1) {  // else no layer reaches the plane
+          int4* a = reinterpret_cast<int4*>(ring + (slot * cy + y) * cx + x);
+          int4* b = reinterpret_cast<int4*>(ring + hi_at + (slot * cy + y) * cx + x);
+          const int4 l4 = *a, h4 = *b;
+          *a = make_int4(0, 0, 0, 0);
+          *b = make_int4(0, 0, 0, 0);
+          const int lo[4] = {l4.x, l4.y, l4.z, l4.w}, hi[4] = {h4.x, h4.y, h4.z, h4.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const long long sum = split ? (long long)hi[k] * 1048576 + lo[k]
+                                        : (long long)(((unsigned long long)(unsigned)hi[k] << 32) | (unsigned)lo[k]);
+            f[k] = __fmul_rn(__ll2float_rn(sum), 9.094947017729282e-13f);  // 2^-40
+            // the physical cells: pad .. n-pad-1
+            if (msum && (unsigned)(ox + x + k - B.pad) < (unsigned)(B.S * q) &&
+                (unsigned)(oy + y - B.pad) < (unsigned)(B.S * q) && (unsigned)(p - B.pad) < (unsigned)(B.S * q))
+              mloc += (unsigned long long)sum;
+          }
+        }
+        if (vec) {
+          __stcs(reinterpret_cast<float4*>(out), make_float4(f[0], f[1], f[2], f[3]));
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (x + k < ex) out[k] = f[k];
+        }
+        slot += gstep;
+        slot = slot >= rd ? slot - rd : slot;
+      }
     }
-  };
-  if (split) visits(std::true_type{});
-  else visits(std::false_type{});
-  __syncthreads();
-  // every cell of the region.  Sums to floats: q * 2^-40 rounded once to FP32 (the int64
-  // to float conversion rounds the exact integer, and scaling by 2^-40 is exact), the value
-  // the FFT's conversion of the int64 mesh gives.
-  auto tofloat = [&](unsigned long long v) {
-    if (split) v = ((v >> 32) << 20) + (v & 0xffffffffull);
-    return __fmul_rn(__ll2float_rn((long long)v), 9.094947017729282e-13f);  // 2^-40
-  };
-  float* base = rho + j * (int64_t)nft * pl + (int64_t)o[2] * pl + (int64_t)o[1] * pr + o[0];
-  if (e[0] == R && e[1] == R && e[2] == RZ && (pr & 3) == 0 && (pl & 3) == 0 &&
-      ((uintptr_t)base & 15) == 0) {
-    // a full region (every region of a class-2 box): four cells per 16-byte store, row and
-    // plane from compile-time divisions
-    constexpr int QX = R / 4;
-    static_assert(R % 4 == 0, "rows of whole float4s");
-    for (int i = tid; i < RZ * R * QX; i += blockDim.x) {
-      const int row = i / QX, qx = i - row * QX;
-      const int z = row / R, y = row - z * R;
-      const unsigned long long* a = &acc[(z * R + y) * R + 4 * qx];
-      const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(a);
-      const ulonglong2 v1 = *reinterpret_cast<const ulonglong2*>(a + 2);
-      __stcs(reinterpret_cast<float4*>(base + (int64_t)z * pl + (int64_t)y * pr) + qx,
-             make_float4(tofloat(v0.x), tofloat(v0.y), tofloat(v1.x), tofloat(v1.y)));
-    }
-    return;
+    done = max(done, upto);
+    __syncthreads();
   }
-  // a partial region: a half warp per row, two cells per 8-byte store (e[0] and the
-  // pitches are even).  z = row / e[1] through a float reciprocal: (row + 0.5) / e[1]
-  // is at least 0.5/e[1] from an integer, far above the rounding error for row < R*R.
-  const int hx = e[0] >> 1, nrow = e[1] * e[2], hl = tid & 15;
-  const float inv_e1 = 1.f / (float)e[1];
-  for (int row = tid >> 4; row < nrow; row += blockDim.x >> 4) {
-    const int z = (int)(((float)row + 0.5f) * inv_e1);
-    const int y = row - z * e[1];
-    if (hl < hx) {
-      const ulonglong2 val = *reinterpret_cast<const ulonglong2*>(&acc[(z * R + y) * R + 2 * hl]);
-      const float2 fv = make_float2(tofloat(val.x), tofloat(val.y));
-      __stcs(reinterpret_cast<float2*>(base + (int64_t)z * pl + (int64_t)y * pr) + hl, fv);
-    }
+  if (msum) {
+    if (fixed) warp_sum_to(mloc, static_cast<unsigned long long*>(msum));
+    else warp_sum_to((double)(long long)mloc * 9.094947017729282e-13, static_cast<double*>(msum));
   }
 }
+
+// The parts of a box: of the splits along x, y and z whose ring fits DEPB_SMEM, the one that
+// an estimate of the time (in rounds of the resident blocks) favours: a layer costs its
+// barriers and dependent loads (DEPB_C0 clocks), its particles (`per_cell` a coarse cell,
+// DEPB_C1 clocks per round of the block's threads) and its write-out (DEPB_C2 per round of 4
+// cells a thread); fewer, larger parts look at fewer particles twice, and few boxes want more
+// parts than fit the ring.
+constexpr double DEPB_C0 = 3000, DEPB_C1 = 4500, DEPB_C2 = 600;
+inline DepBox dep_box(int S, int halo, int q, int pad, int iapm, int64_t nbox, double per_cell, int nsm) {
+  DepBox B{};
+  B.S = S;
+  B.halo = halo;
+  B.q = q;
+  B.pad = pad;
+  B.iapm = iapm;
+  B.n = S * q + 2 * pad;
+  const int nl = S + 2 * halo;
+  double best = -1;
+  int lastx = 0;
+  for (int nx = 1; nx <= 32; ++nx) {
+    const int cx = ((B.n + nx - 1) / nx + 3) / 4 * 4, ncx = (B.n + cx - 1) / cx;
+    if (cx == lastx || (cx < 8 && nx > 1 && best >= 0)) continue;
+    lastx = cx;
+    int lasty = 0;
+    for (int ny = 1, tried = 0; ny <= B.n && tried < 4; ++ny) {
+      const int cy = (B.n + ny - 1) / ny, ncy = (B.n + cy - 1) / cy;
+      if (cy == lasty || (int64_t)cx * cy * (q + 2) * 8 > DEPB_SMEM || cy > 28 * q) continue;
+      lasty = cy;
+      ++tried;
+      const double kx = std::min(nl, (cx + 1) / q + 2), ky = std::min(nl, (cy + 1) / q + 2);
+      const double layer = DEPB_C0 + DEPB_C1 * std::max(1.0, kx * ky * per_cell / DEPB_T) +
+                           DEPB_C2 * std::max(1.0, (double)cx * cy * q / (4 * DEPB_T));
+      for (int lz = nl; lz >= 1; lz = lz > 1 ? (lz + 1) / 2 : 0) {  // layers a part
+        const int cz = std::min(B.n, lz * q), ncz = (B.n + cz - 1) / cz;
+        const double blocks = (double)nbox * ncx * ncy * ncz, slots = 2.0 * nsm;
+        const double rounds = blocks <= 8 * slots ? std::ceil(blocks / slots) : blocks / slots;
+        const double cost = rounds * std::min(nl, lz + 2) * layer;
+        if (best < 0 || cost < best) {
+          best = cost;
+          B.cx = cx;
+          B.cy = cy;
+          B.cz = cz;
+          B.ncx = ncx;
+          B.ncy = ncy;
+          B.ncz = ncz;
+        }
+      }
+    }
+  }
+  return B;
+}
+inline size_t dep_box_smem(const DepBox& B) { return (size_t)B.cx * B.cy * (B.q + 2) * 8; }
 
 // =================================================================================
 // Force from potential (particle_mesh.f90:224-247, kick.f90:839-862) and max |F|^2.

@@ -1788,18 +1788,18 @@ struct PPi {
   }
 };
 
-// The plain form: one thread per particle over the coarse cells its range reaches, reading
-// the candidates' codes.  Candidates go four at a time as independent chains; pairs in range
+// The plain form: one thread per particle of the cells of at most heavy_t particles, over the
+// coarse cells its range reaches, reading the candidates' codes (fuller cells go to
+// k_ppq_heavy).  Candidates go four at a time as independent chains; pairs in range
 // are kept in the thread's own shared-memory column and added with PPi::accum in candidate
 // order when it may run full and at the end, so that the lanes of a warp evaluate their
-// pairs together (128^3 particles at 8 a cell: 0.76 -> 0.42 ms; at 64 a cell with cells of up
-// to 4e3: 14.5 -> 12.3 ms, bound by the lanes' different neighbour cells).
+// pairs together (128^3 particles at 8 a cell: 0.76 -> 0.42 ms).
 constexpr int PP_T = 128, PP_H = 8, PP_U = 4;
 template <bool FAST, typename CODE>
 __global__ void __launch_bounds__(PP_T) k_pp(Geo G, int64_t np, const CODE* __restrict__ xp,
                                              const int32_t* __restrict__ pcell, const int64_t* __restrict__ cstart,
                                              const int32_t* __restrict__ ires, float* __restrict__ vp,
-                                             const StepDev* __restrict__ sd, float* f2max, float* vmax,
+                                             const StepDev* __restrict__ sd, int heavy_t, float* f2max, float* vmax,
                                              unsigned long long* npairs, unsigned long long* ncand,
                                              const unsigned* __restrict__ abort) {
   __shared__ float4 hb[PP_H][PP_T];
@@ -1810,7 +1810,7 @@ __global__ void __launch_bounds__(PP_T) k_pp(Geo G, int64_t np, const CODE* __re
   int c = 0;
   if (live) {
     c = pcell[ip];
-    live = owned_cell(G, c);
+    live = owned_cell(G, c) && cstart[c + 1] - cstart[c] <= heavy_t;
   }
   float f2 = 0.f, av[3] = {0.f, 0.f, 0.f};
   PPi P;

@@ -12,8 +12,9 @@
 //     cells' particles in shared memory in chunks of J and tests its B particles against
 //     each chunk.  The queue is ordered by occupancy, largest first (log2 buckets), so the
 //     long items start first and the tail is short.
-// Both paths read the candidates' in-cell offsets, decoded once per step into a float4
-// array (k_ppq_prep), test candidates four at a time as independent chains, defer the
+// The light path reads the candidates' in-cell offsets, decoded once per step into a float4
+// array (k_ppq_prep); the heavy path decodes them as it stages them.  Both test candidates
+// four at a time as independent chains, defer the
 // pairs in range to a per-thread shared-memory column and add them in candidate order,
 // so each particle's pairs are summed with the same operations in the same order and the
 // force does not depend on (T, B, J): the autotuner (cube_gpu.cu, pp_tune) picks the
@@ -47,6 +48,15 @@ __device__ __forceinline__ float ppq_apply(const PPi& P, int64_t ip, const float
     av[d] = fabsf(v);
   }
   return sumsq3(f1[0], f1[1], f1[2]);
+}
+
+// In-cell offset of one particle from its codes: (u + 0.5) * step with step = x_res*ratio_cs a
+// power of two, exact as in k_ppq_prep.
+template <typename CODE>
+__device__ __forceinline__ float4 ppq_offset(const CODE* __restrict__ xp, int64_t ip, float step) {
+  const CODE* c = xp + 3 * ip;
+  return make_float4(fmaf((float)c[0], step, 0.5f * step), fmaf((float)c[1], step, 0.5f * step),
+                     fmaf((float)c[2], step, 0.5f * step), 0.f);
 }
 
 __device__ __forceinline__ int ppq_iapm(const Geo& G, const int g[3], const int32_t* ires) {
@@ -231,10 +241,12 @@ __device__ __forceinline__ int ppq_code(const PPi& P) {
 // arbitrary).  The items of B consecutive entries then hold one or two codes, so that a
 // block stages, and a warp computes, only the cells their particles reach.  Each
 // particle's sums do not depend on the item or thread that computes them.
+template <typename CODE>
 __global__ void __launch_bounds__(256) k_ppq_sort_codes(Geo G, const int32_t* __restrict__ hlist,
                                                         const int* __restrict__ q, const int64_t* __restrict__ cstart,
                                                         const int32_t* __restrict__ ires,
-                                                        const float4* __restrict__ pfin, int32_t* __restrict__ hperm) {
+                                                        const CODE* __restrict__ xp, int32_t* __restrict__ hperm) {
+  const float step = (float)(G.x_res * (double)G.rcs);
   __shared__ int cnt[64];
   const int nh = q[64];
   for (int h = blockIdx.x; h < nh; h += gridDim.x) {
@@ -248,7 +260,7 @@ __global__ void __launch_bounds__(256) k_ppq_sort_codes(Geo G, const int32_t* __
     __syncthreads();
     for (int64_t ip = s0 + threadIdx.x; ip < e0; ip += blockDim.x) {
       PPi P;
-      P.init(G, g, pfin[ip], iapm);
+      P.init(G, g, ppq_offset(xp, ip, step), iapm);
       atomicAdd(&cnt[ppq_code(P)], 1);
     }
     __syncthreads();
@@ -266,7 +278,7 @@ __global__ void __launch_bounds__(256) k_ppq_sort_codes(Geo G, const int32_t* __
     __syncthreads();
     for (int64_t ip = s0 + threadIdx.x; ip < e0; ip += blockDim.x) {
       PPi P;
-      P.init(G, g, pfin[ip], iapm);
+      P.init(G, g, ppq_offset(xp, ip, step), iapm);
       hperm[s0 + atomicAdd(&cnt[ppq_code(P)], 1)] = (int32_t)ip;
     }
   }
@@ -290,9 +302,10 @@ __host__ __device__ inline size_t ppq_heavy_smem(int B, int J) {
   return (size_t)PPH_H * B * sizeof(float4) + (size_t)3 * ppq_chunk_pitch(J) * sizeof(float);
 }
 
+template <typename CODE>
 __global__ void k_ppq_heavy(Geo G, const int32_t* __restrict__ hlist, const int* __restrict__ hpre, int* q,
                             const int64_t* __restrict__ cstart, const int32_t* __restrict__ ires,
-                            const float4* __restrict__ pfin, const int32_t* __restrict__ hperm, const float* vin,
+                            const CODE* __restrict__ xp, const int32_t* __restrict__ hperm, const float* vin,
                             float* vout, const StepDev* __restrict__ sd, int J, float* f2max, float* vmax,
                             unsigned long long* npairs, unsigned long long* ncand, const unsigned* __restrict__ abort) {
   extern __shared__ float4 sj[];  // the deferred pairs [PPH_H][B], then x, y, z of JP candidates
@@ -305,6 +318,7 @@ __global__ void k_ppq_heavy(Geo G, const int32_t* __restrict__ hlist, const int*
   const bool aborted = abort && *abort;
   const int nh = q[64], nitems = q[65];
   const float mass_scale = sd->pp_mass, v_scale = sd->pp_vscale;
+  const float step = (float)(G.x_res * (double)G.rcs);
   float f2m = 0.f, av[3] = {0.f, 0.f, 0.f};
   unsigned long long tp = 0, tc = 0;
   for (;;) {
@@ -328,7 +342,7 @@ __global__ void k_ppq_heavy(Geo G, const int32_t* __restrict__ hlist, const int*
     int g[3];
     cell_coords(G, c, g[0], g[1], g[2]);
     PPi P;
-    P.init(G, g, pfin[live ? ip : s0], ppq_iapm(G, g, ires));
+    P.init(G, g, ppq_offset(xp, ip, step), ppq_iapm(G, g, ires));
     int nh = 0;
     auto flush = [&]() {
 #pragma unroll 1
@@ -355,7 +369,7 @@ __global__ void k_ppq_heavy(Geo G, const int32_t* __restrict__ hlist, const int*
             const int cnt = (int)((e - j0) < (int64_t)J ? (e - j0) : (int64_t)J);
             __syncthreads();
             for (int k = threadIdx.x; k < cnt; k += B) {
-              const float4 p = pfin[j0 + k];
+              const float4 p = ppq_offset(xp, j0 + k, step);
               sx[k] = p.x;
               sy[k] = p.y;
               sz[k] = p.z;

@@ -1451,7 +1451,7 @@ static int enqueue_kick_a(cube_ctx* c) {
     const int64_t n3 = (int64_t)n * n * n;
     if (foff + (size_t)n3 * sizeof(float4) <= c->arena_bytes) {
       float4* force = reinterpret_cast<float4*>(reinterpret_cast<char*>(c->arena) + foff);
-      LAUNCH(c, K_INT_PM1, 1, k_force_pm1<<<nblk(n3), 256, 0, c->s>>>(n, phi, m.pt.pf, m.pt.plf, force));
+      LAUNCH(c, K_INT_PM1, 1, k_force_pm1<<<force_grid(n), FORCE_T, 0, c->s>>>(n, phi, m.pt.pf, m.pt.plf, force));
       LAUNCH(c, K_INT_PM1, 1, k_interp_pm1_force<<<nblk(npo), 256, 0, c->s>>>(G, npo, xpo, pco, force, vpo, c->sd));
     } else {
       LAUNCH(c, K_INT_PM1, 1, k_interp_pm1<<<nblk(npo), 256, 0, c->s>>>(G, npo, xpo, pco, phi, vpo, c->sd, m.pt.pf, m.pt.plf));
@@ -2720,17 +2720,63 @@ int noalloc_scratch(unsigned char** out) {
   return 0;
 }
 
-// Particle -> cell index from the cell starts; indices at or beyond np are not written,
-// so a rhoc that does not sum to np cannot write past the scratch.  A negative count
-// (cstart decreasing) raises *bad, which the host turns into CUBE_E_COUNT.
-__global__ void k_na_fill_pcell(const int64_t* __restrict__ cstart, int64_t ncells, int64_t np,
-                                int32_t* __restrict__ pcell, unsigned* __restrict__ bad) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncells) return;
-  if (cstart[c + 1] < cstart[c]) atomicOr(bad, 1u);
-  const int64_t b = cstart[c] > 0 ? cstart[c] : 0;
-  const int64_t e = cstart[c + 1] < np ? cstart[c + 1] : np;
-  for (int64_t i = b; i < e; ++i) pcell[i] = (int32_t)c;
+// The preparation of the allocation-free density in two kernels, one block per SCAN_TILE cells
+// (at most 128): every launch and copy of a call this small costs as much as its work, and
+// the cell scan, the clears and the particle -> cell index were eight of them.
+// First: the tile's count and its smallest count, and the accumulator cleared.
+__global__ void k_na_tiles(const int32_t* __restrict__ in, int64_t n, int64_t* __restrict__ tile_sums,
+                           int32_t* __restrict__ tile_min, unsigned long long* __restrict__ acc64,
+                           float* __restrict__ acc32) {
+  const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_I;
+  int64_t s = 0;
+  int neg = 0;
+#pragma unroll
+  for (int i = 0; i < SCAN_I; ++i)
+    if (base + i < n) {
+      const int32_t v = in[base + i];
+      s += v;
+      neg |= v < 0;
+      if (acc64) acc64[base + i] = 0ull;
+      else acc32[base + i] = 0.f;
+    }
+  int64_t tot;
+  block_excl_scan(s, &tot);
+  neg = __syncthreads_or(neg);
+  if (threadIdx.x == 0) {
+    tile_sums[blockIdx.x] = tot;
+    tile_min[blockIdx.x] = neg;
+  }
+}
+
+// Second: particle -> cell index from the running counts; indices at or beyond np are not
+// written, and particles beyond the counts go to cell 0, so a rhoc that does not sum to np
+// cannot read or write past the scratch.  status: the total count, and whether one was
+// negative, which the host turns into CUBE_E_COUNT.
+__global__ void __launch_bounds__(SCAN_T) k_na_index(const int32_t* __restrict__ in, int64_t n, int64_t np,
+                                                     const int64_t* __restrict__ tile_sums,
+                                                     const int32_t* __restrict__ tile_min, int ntiles,
+                                                     int64_t* __restrict__ status, int32_t* __restrict__ pcell) {
+  // a block takes SCAN_T cells, one per thread; ntiles is at most SCAN_T
+  const int64_t c0 = (int64_t)blockIdx.x * SCAN_T, c = c0 + threadIdx.x;
+  const int tile = (int)(c0 / SCAN_TILE), t = (int)threadIdx.x;
+  const int64_t v = t < ntiles ? tile_sums[t] : 0;
+  int64_t total, before, at = 0;
+  block_excl_scan(v, &total);
+  int64_t lead = t < tile ? v : 0;  // the tiles before, and the cells of this tile before c0
+  for (int64_t i = (int64_t)tile * SCAN_TILE + t; i < c0; i += SCAN_T) lead += in[i];
+  block_excl_scan(lead, &before);
+  const int neg = __syncthreads_or(t < ntiles ? tile_min[t] : 0);
+  if (blockIdx.x == 0 && t == 0) {
+    status[0] = total;
+    status[1] = neg;
+  }
+  const int32_t cnt = c < n ? in[c] : 0;
+  int64_t tot;
+  at = block_excl_scan(cnt, &tot) + before;
+  const int64_t b = at > 0 ? at : 0, e = at + cnt < np ? at + cnt : np;
+  for (int64_t j = b; j < e; ++j) pcell[j] = (int32_t)c;
+  for (int64_t j = (neg || total < 0 ? 0 : total) + (int64_t)blockIdx.x * SCAN_T + t; j < np; j += (int64_t)gridDim.x * SCAN_T)
+    pcell[j] = 0;
 }
 
 // Fixed-point weight sums -> density in mass units, rounded as cube_gpu_captured does.
@@ -2775,14 +2821,16 @@ extern "C" int cube_gpu_pm1_density_noalloc(const cube_params* p, const void* xp
   const bool fixed = p->deposit_mode == CUBE_DEPOSIT_FIXED;
   const int nc = G.nc;
   const int64_t n3 = G.ncells;
-  // The array keeps the previous call's contents: clear the accumulator and the cell
-  // indices (the scan overwrites every cell start and tile sum it reads).
-  if (fixed) CK(cudaMemsetAsync(acc, 0, n3 * 8, s));
-  else CK(cudaMemsetAsync(rho, 0, n3 * 4, s));
-  if (np > 0) CK(cudaMemsetAsync(pcell, 0, np * 4, s));
-  CK(cudaMemsetAsync(bad, 0, sizeof(unsigned), s));
-  exclusive_scan(rhoc, cstart, n3, tmp, s);
-  k_na_fill_pcell<<<nblk(n3), 256, 0, s>>>(cstart, n3, np, pcell, bad);
+  // The array keeps the previous call's contents: the first kernel clears the accumulator; the
+  // second writes every cell index that the deposit reads, and the tile sums and the status
+  // are written before they are read.  A negative count leaves indices unwritten (the last
+  // call's, all cells of the scratch): the result is an error then, and the deposit is
+  // bounded by np and by those cells.
+  const unsigned tiles = nblk(n3, SCAN_TILE);
+  int64_t* status = reinterpret_cast<int64_t*>(bad);
+  int32_t* tile_min = reinterpret_cast<int32_t*>(cstart);
+  k_na_tiles<<<tiles, SCAN_T, 0, s>>>(rhoc, n3, tmp, tile_min, fixed ? reinterpret_cast<unsigned long long*>(acc) : nullptr, rho);
+  k_na_index<<<nblk(n3, SCAN_T), SCAN_T, 0, s>>>(rhoc, n3, np, tmp, tile_min, (int)tiles, status, pcell);
   if (np > 0) {
     if (fixed) k_deposit_pm1<true><<<nblk(np), 256, 0, s>>>(G, np, xp, pcell, acc, nc, (int64_t)nc * nc, nullptr);
     else k_deposit_pm1<false><<<nblk(np), 256, 0, s>>>(G, np, xp, pcell, rho, nc, (int64_t)nc * nc, nullptr);
@@ -2791,11 +2839,10 @@ extern "C" int cube_gpu_pm1_density_noalloc(const cube_params* p, const void* xp
   else k_na_scale<<<nblk(n3), 256, 0, s>>>(rho, n3, G.mass_p);
   CK(cudaGetLastError());
   // every particle must belong to a cell (drift.f90:139-143 checks the same sum)
-  int64_t total = -1;
-  unsigned negative = 0;
-  CK(cudaMemcpyAsync(&total, cstart + n3, sizeof total, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&negative, bad, sizeof negative, cudaMemcpyDeviceToHost, s));
+  int64_t seen[2] = {-1, 0};
+  CK(cudaMemcpyAsync(seen, status, sizeof seen, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
+  const int64_t total = seen[0], negative = seen[1];
   if (negative) return fail(CUBE_E_COUNT, "rhoc holds a negative count");
   if (total != np) {
     char msg[160];
@@ -2876,7 +2923,7 @@ extern "C" int cube_gpu_power(cube_ctx* c, const cube_power_in* in, float* xi, i
   }
   float* mesh = reinterpret_cast<float*>(base);
   long long* acc = reinterpret_cast<long long*>(base + mbytes);
-  const int nred = 4 * 148;
+  const int nred = 8 * 148;
   const size_t nbins4 = 4 * (size_t)(nbin + 1), nbins3 = 3 * (size_t)(nbin + 1);
   void* small = nullptr;
   const size_t sbytes = (nred + 1 + nbins4 + nbins3) * sizeof(double) + 2 * sizeof(int);
@@ -2921,7 +2968,7 @@ extern "C" int cube_gpu_power(cube_ctx* c, const cube_power_in* in, float* xi, i
   const double mean = rho8 / (double)nw / (double)nw / (double)nw;
   const int mm0[2] = {0x7fffffff, (int)0x80000000};
   PK_CK(cudaMemcpyAsync(mm, mm0, sizeof(mm0), cudaMemcpyHostToDevice, c->s));
-  LAUNCH(c, K_PK_DEP, 1, k_pk_delta<<<nred, 256, 0, c->s>>>(mesh, nw, pt.pr, pt.plr, mean, mm));
+  LAUNCH(c, K_PK_DEP, 1, k_pk_delta<<<nred, 256, 0, c->s>>>(mesh, nw, pt.pr, pt.plr, 1.0 / mean, mm));
   if (delta) {
     if (pt.pr == nw)  // plane-compact: each plane's rows are contiguous
       PK_CK(cudaMemcpy2DAsync(delta, (size_t)nw * nw * 4, mesh, pt.psb, (size_t)nw * nw * 4, nw, cudaMemcpyDeviceToHost, c->s));
@@ -3033,8 +3080,7 @@ int dpm_force_mesh(cube_dpm* d, const float* x, int64_t np) {
   CK(cudaMemsetAsync(d->mesh, 0, mesh_bytes(c, n, 1, false), c->s));
   if (np > 0) k_dpm_deposit<<<nblk(np), 256, 0, c->s>>>(n, np, x, d->mass, d->mesh, d->pt.pr, d->pt.plr);
   launch_fft(c, n, 1, d->mesh, false, 1.f, d->mesh, reinterpret_cast<float2*>(d->mesh), c->green1, (float)n, 3, 1);
-  const int64_t n3 = (int64_t)n * n * n;
-  k_force_pm1<<<nblk(n3), 256, 0, c->s>>>(n, d->mesh, d->pt.pf, d->pt.plf, d->fm);
+  k_force_pm1<<<force_grid(n), FORCE_T, 0, c->s>>>(n, d->mesh, d->pt.pf, d->pt.plf, d->fm);
   c->launches += 7;
   return 0;
 }
@@ -3160,7 +3206,7 @@ int cube_dpm_force_vjp(cube_dpm* d, const float* x, int64_t np, const float* u, 
   if (rc) return rc;
   CK(cudaMemsetAsync(d->lam, 0, n3 * sizeof(float4), c->s));
   if (np > 0) k_dpm_deposit_vec<<<nblk(np), 256, 0, c->s>>>(n, np, x, u, d->lam);
-  k_dpm_grad_t<<<nblk(n3), 256, 0, c->s>>>(n, d->lam, d->mesh, d->pt.pr, d->pt.plr);
+  k_dpm_grad_t<<<force_grid(n), FORCE_T, 0, c->s>>>(n, d->lam, d->mesh, d->pt.pr, d->pt.plr);
   launch_fft(c, n, 1, d->mesh, false, 1.f, d->mesh, reinterpret_cast<float2*>(d->mesh), c->green1, (float)n, 3, 1);
   if (np > 0)
     k_dpm_grad_gather<<<nblk(np), 256, 0, c->s>>>(n, np, x, u, d->fm, d->mesh, d->pt.pf, d->pt.plf, d->mass, gx);

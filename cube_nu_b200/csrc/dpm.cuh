@@ -135,20 +135,20 @@ __global__ void k_dpm_deposit_vec(int n, int64_t np, const float* __restrict__ x
 
 // s(c) = (grad_h^T lamF)(c) = sum_d sum_o w_o lamF_d(c - o e_d), o in {-2,-1,1,2}, the
 // transpose of the 4-point gradient; written into a mesh with row pitch pr, plane pl.
-__global__ void k_dpm_grad_t(int n, const float4* __restrict__ lam, float* __restrict__ s, int pr, int64_t pl) {
-  const unsigned un = (unsigned)n, i = blockIdx.x * blockDim.x + threadIdx.x;  // n < 1626
-  if (i >= un * un * un) return;
-  const unsigned zy = i / un;
-  const int x = (int)(i - zy * un), z = (int)(zy / un), y = (int)(zy - (unsigned)z * un);
+// Grid of force_grid.
+__global__ void __launch_bounds__(FORCE_T) k_dpm_grad_t(int n, const float4* __restrict__ lam, float* __restrict__ s,
+                                                        int pr, int64_t pl) {
+  const int x = blockIdx.x * FORCE_T + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
+  if (x >= n) return;
   const float w[4] = {(CUBE_W_ALPHA - 1.f) / 4.f, -CUBE_W_ALPHA / 2.f, CUBE_W_ALPHA / 2.f, (1.f - CUBE_W_ALPHA) / 4.f};
   const int o[4] = {-2, -1, 1, 2};
-  auto L = [&](int a, int b, int c) { return __ldg(&lam[((int64_t)c * n + b) * n + a]); };
+  auto L = [&](int a, int b, int c) { return reinterpret_cast<const float*>(lam + ((int64_t)c * n + b) * n + a); };
   float t = 0.f;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    t += w[k] * L(wrap1(x - o[k], n), y, z).x;
-    t += w[k] * L(x, wrap1(y - o[k], n), z).y;
-    t += w[k] * L(x, y, wrap1(z - o[k], n)).z;
+    t += w[k] * __ldg(L(wrap1(x - o[k], n), y, z));
+    t += w[k] * __ldg(L(x, wrap1(y - o[k], n), z) + 1);
+    t += w[k] * __ldg(L(x, y, wrap1(z - o[k], n)) + 2);
   }
   s[(int64_t)z * pl + (int64_t)y * pr + x] = t;
 }

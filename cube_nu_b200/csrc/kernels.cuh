@@ -1456,21 +1456,22 @@ __global__ void k_interp_pm1(Geo G, int64_t np, const void* __restrict__ xp, con
 // (particle_mesh.f90:224-247): at every coarse cell j (0-based, periodic) the three
 // components grad4(phi(j-2), phi(j-1), phi(j+1), phi(j+2)), with the same FP32
 // operations as tsc_gather_force, stored as float4 (fx, fy, fz, 0), x fastest.
-// Cell indices in 32 bits (contexts hold fewer than 2^32 cells) and wraps by comparison: with
-// 64-bit divisions it took 0.24 ms at 256^3, five times the write of the force mesh.
-__global__ void __launch_bounds__(256) k_force_pm1(int nc, const float* __restrict__ phi, int pf, int64_t pl,
-                                                   float4* __restrict__ force) {
-  const unsigned n = (unsigned)nc, i = blockIdx.x * 256u + threadIdx.x;
-  if (i >= n * n * n) return;
-  const unsigned zy = i / n;
-  const int x = (int)(i - zy * n), z = (int)(zy / n), y = (int)(zy - (unsigned)z * n);
-  const int64_t row = (int64_t)z * pl + (int64_t)y * pf, xl = (int64_t)z * pl + x;
-  const float* ph = phi;
-  auto X = [&](int d) { return __ldg(&ph[row + wrap1(x + d, nc)]); };
-  auto Y = [&](int d) { return __ldg(&ph[xl + (int64_t)wrap1(y + d, nc) * pf]); };
-  auto Z = [&](int d) { return __ldg(&ph[(int64_t)wrap1(z + d, nc) * pl + (int64_t)y * pf + x]); };
-  force[i] = make_float4(grad4(X(-2), X(-1), X(1), X(2)), grad4(Y(-2), Y(-1), Y(1), Y(2)),
-                         grad4(Z(-2), Z(-1), Z(1), Z(2)), 0.f);
+// Grid (blocks along x, y, z) of FORCE_T cells along x: with a flat index and 64-bit divisions
+// it took 0.24 ms at 256^3, five times the write of the force mesh.
+constexpr int FORCE_T = 128;
+inline dim3 force_grid(int nc) { return dim3((unsigned)((nc + FORCE_T - 1) / FORCE_T), (unsigned)nc, (unsigned)nc); }
+__global__ void __launch_bounds__(FORCE_T) k_force_pm1(int nc, const float* __restrict__ phi, int pf, int64_t pl,
+                                                       float4* __restrict__ force) {
+  const int x = blockIdx.x * FORCE_T + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
+  if (x >= nc) return;
+  const float* row = phi + (int64_t)z * pl + (int64_t)y * pf;
+  const float* col = phi + (int64_t)z * pl + x;
+  const float* line = phi + (int64_t)y * pf + x;
+  auto X = [&](int d) { return __ldg(row + wrap1(x + d, nc)); };
+  auto Y = [&](int d) { return __ldg(col + (int64_t)wrap1(y + d, nc) * pf); };
+  auto Z = [&](int d) { return __ldg(line + (int64_t)wrap1(z + d, nc) * pl); };
+  force[((int64_t)z * nc + y) * nc + x] = make_float4(grad4(X(-2), X(-1), X(1), X(2)), grad4(Y(-2), Y(-1), Y(1), Y(2)),
+                                                      grad4(Z(-2), Z(-1), Z(1), Z(2)), 0.f);
 }
 
 // PM1 interpolation + kick from the force mesh: the 27 TSC points of a particle are the

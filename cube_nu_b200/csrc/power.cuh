@@ -114,19 +114,27 @@ __device__ __forceinline__ int float_order_key(float f) {
   return i >= 0 ? i : i ^ 0x7fffffff;
 }
 
-// delta = rho/mean - 1 in place (cicpower.f90:180: real(4)/real(8) - 1 -> real(4)),
-// with min/max keys in mm[0], mm[1].
-__global__ void k_pk_delta(float* __restrict__ mesh, int nw, int pr, int64_t pl, double mean, int* __restrict__ mm) {
-  const unsigned rows = (unsigned)nw * (unsigned)nw, warps = gridDim.x * 8u;  // blockDim = 256, a row per warp
+// delta = rho/mean - 1 in place (cicpower.f90:180: real(4)/real(8) - 1 -> real(4), the
+// division as a product with the reciprocal in double), with min/max keys in mm[0], mm[1].
+// blockDim = 256, a row per warp, 4 values in flight per lane.
+__global__ void k_pk_delta(float* __restrict__ mesh, int nw, int pr, int64_t pl, double inv_mean, int* __restrict__ mm) {
+  const unsigned rows = (unsigned)nw * (unsigned)nw, warps = gridDim.x * 8u;
   float lo = 3.0e38f, hi = -3.0e38f;
   for (unsigned row = blockIdx.x * 8u + (threadIdx.x >> 5); row < rows; row += warps) {
     const unsigned z = row / (unsigned)nw, y = row - z * (unsigned)nw;
     float* m = mesh + (int64_t)z * pl + (int64_t)y * pr;
-    for (int x = threadIdx.x & 31; x < nw; x += 32) {
-      const float d = __double2float_rn(__dsub_rn(__ddiv_rn((double)m[x], mean), 1.0));
-      m[x] = d;
-      lo = fminf(lo, d);
-      hi = fmaxf(hi, d);
+    for (int x0 = threadIdx.x & 31; x0 < nw; x0 += 128) {
+      float r[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) r[k] = x0 + 32 * k < nw ? m[x0 + 32 * k] : 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (x0 + 32 * k < nw) {
+          const float d = __double2float_rn(__fma_rn((double)r[k], inv_mean, -1.0));
+          m[x0 + 32 * k] = d;
+          lo = fminf(lo, d);
+          hi = fmaxf(hi, d);
+        }
     }
   }
   for (int o = 16; o > 0; o >>= 1) {

@@ -413,7 +413,7 @@ Pitch pitch_of(const cube_ctx* c, int n, bool fixed) {
   const int64_t rb = fixed ? 8 : 4, nh = n / 2 + 1;
   Pitch p;
   if (fused_layout(c, n)) {
-    p.pc = (int)(nh + 1) / 2 * 2;
+    p.pc = f2::plane_pc(n);
     p.psb = std::max<int64_t>((int64_t)n * n * rb, (int64_t)n * p.pc * 8);
     p.pr = n;
     p.pf = n;
@@ -496,22 +496,22 @@ void fft2_run(cube_ctx* c, int64_t nbox, const void* real_in, bool fixed, float 
       if (fixed) {
         smem_optin(f2::k_fxy3_r2c<N, R1, R2, long long>, smf);
         LAUNCH(c, kx, 1, f2::k_fxy3_r2c<N, R1, R2, long long><<<planes, f2::PlaneShape<N, R1, R2>::THREADS, smf, c->s>>>(
-                             (const long long*)real_in, ck, tw, scale, pt.pr, pt.pc, pt.plr, pt.plc));
+                             (const long long*)real_in, ck, tw, scale, pt.plr, pt.plc));
       } else {
         smem_optin(f2::k_fxy3_r2c<N, R1, R2, float>, smf);
         LAUNCH(c, kx, 1, f2::k_fxy3_r2c<N, R1, R2, float><<<planes, f2::PlaneShape<N, R1, R2>::THREADS, smf, c->s>>>(
-                             (const float*)real_in, ck, tw, scale, pt.pr, pt.pc, pt.plr, pt.plc));
+                             (const float*)real_in, ck, tw, scale, pt.plr, pt.plc));
       }
       using Z = f2::ZLoop<N, R1, R2>;
       const int lines = N * Z::NCG, ns = f2::fz_loop_split(lines, c->nsm * Z::MINB, nbox);
       auto zl = f2::k_fz_loop<N, R1, R2>;
       smem_optin(zl, Z::SMEM);
-      LAUNCH(c, kz, 1, zl<<<(unsigned)(lines * ns), Z::THREADS, Z::SMEM, c->s>>>(ck, green, tw, pt.pc, pt.plc, nbox, ns, lo,
+      LAUNCH(c, kz, 1, zl<<<(unsigned)(lines * ns), Z::THREADS, Z::SMEM, c->s>>>(ck, green, tw, pt.plc, nbox, ns, lo,
                                                                                  hi));
       smem_optin(f2::k_fyx3_c2r<N, R1, R2>, smi);
       const unsigned cplanes = (unsigned)(nbox * (hi - lo));
       LAUNCH(c, kc, 1, f2::k_fyx3_c2r<N, R1, R2><<<cplanes, f2::PlaneShape<N, R1, R2>::THREADS, smi, c->s>>>(
-                           ck, phi_out, tw, inv, pt.pc, pt.pf, pt.plc, pt.plf, lo, hi));
+                           ck, phi_out, tw, inv, pt.plc, pt.plf, lo, hi));
       return;
     }
   }
@@ -589,7 +589,7 @@ void fft2_forward(cube_ctx* c, float* real, const Pitch& pt, int cls) {
       const size_t smf = f2::Plane3Sm<N>::FWD;
       smem_optin(f2::k_fxy3_r2c<N, R1, R2, float>, smf);
       LAUNCH(c, cls, 1, f2::k_fxy3_r2c<N, R1, R2, float><<<(unsigned)N, f2::PlaneShape<N, R1, R2>::THREADS, smf, c->s>>>(
-                            real, ck, tw, 1.f, pt.pr, pt.pc, pt.plr, pt.plc));
+                            real, ck, tw, 1.f, pt.plr, pt.plc));
       LAUNCH(c, cls, 1, f2::k_fcol3<N, R1, R2, 2, 0><<<gc, W * T, smc, c->s>>>(ck, tw, W, pt.pc, pt.plc));
       return;
     }

@@ -361,6 +361,9 @@ __global__ void __launch_bounds__(FcolBounds<N, TPS<R1, R2>::T>::MAXT, FcolBound
   }
 }
 
+// Row pitch of the half spectrum in the plane-compact layout; real rows have N values.
+__host__ __device__ constexpr int plane_pc(int N) { return (N / 2 + 2) / 2 * 2; }
+
 // ---------------------------------------------------------------------------------
 // z pass with Green multiply for the plane sizes (N <= 144): forward z DFT, Green multiply,
 // inverse, with a block kept on one line y and one group of columns while it walks the boxes, so the
@@ -393,7 +396,7 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 
 template <int N, int R1, int R2>
 __global__ void __launch_bounds__(ZLoop<N, R1, R2>::THREADS, ZLoop<N, R1, R2>::MINB)
-    k_fz_loop(float2* __restrict__ c, const float* __restrict__ green, const float2* __restrict__ gtw, int pc, int64_t plc,
+    k_fz_loop(float2* __restrict__ c, const float* __restrict__ green, const float2* __restrict__ gtw, int64_t plc,
               int64_t nbox, int nsplit, int lo, int hi) {
   using Z = ZLoop<N, R1, R2>;
   constexpr int NH = Z::NH, WC = Z::WC, COLS = Z::COLS;
@@ -410,7 +413,7 @@ __global__ void __launch_bounds__(ZLoop<N, R1, R2>::THREADS, ZLoop<N, R1, R2>::M
     const int z = i / COLS, q = i - z * COLS;
     gr[i] = q < ncol ? green[((int64_t)z * N + y) * NH + kx0 + q] : 0.f;
   }
-  auto base = [&](int64_t b) { return c + b * (int64_t)N * plc + (int64_t)y * pc + kx0; };
+  auto base = [&](int64_t b) { return c + b * (int64_t)N * plc + y * plane_pc(N) + kx0; };
   auto issue = [&](int64_t b, int st) {
     const float2* src = base(b);
     float2* dst = stg + st * N * WC;
@@ -686,9 +689,9 @@ __device__ __forceinline__ int skew(int k1, int n2) {
 
 template <int N, int R1, int R2, typename IN>
 __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, R1, R2>::MINB) k_fxy3_r2c(const IN* __restrict__ r, float2* __restrict__ c,
-                                                               const float2* __restrict__ gtw, float scale, int pr,
-                                                               int pc, int64_t plr, int64_t plc) {
-  constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1, NP = N / 2;
+                                                               const float2* __restrict__ gtw, float scale, int64_t plr,
+                                                               int64_t plc) {
+  constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1, NP = N / 2, PC = plane_pc(N);
   static_assert(T <= 16, "two sequences per warp");
   extern __shared__ float2 sm[];
   float2* tw = sm;
@@ -712,7 +715,7 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
 #pragma unroll
         for (int n1 = 0; n1 < R1; ++n1) {
           const int x = R2 * n1 + t;
-          const IN a = rp[(2 * p) * pr + x], b = rp[(2 * p + 1) * pr + x];
+          const IN a = rp[(2 * p) * N + x], b = rp[(2 * p + 1) * N + x];
           float fa, fb;
           if (sizeof(IN) == 8) {
             fa = (float)((double)(long long)a * 9.094947017729282e-13);
@@ -756,8 +759,8 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
       const bool selfc = (kx == 0) || (2 * kx == N);
       const int st = selfc ? 1 : N;
       // offsets from Z (S follows Z): slot s at Z[lo + s*st] for s < NP, else Z[hi + s*st]
-      const int64_t lo = selfc ? (int64_t)NP * N + (kx ? N : 0) : (int64_t)kx;
-      const int64_t hi = selfc ? lo : (int64_t)kc - (int64_t)NP * N;
+      const int lo = selfc ? NP * N + (kx ? N : 0) : kx;
+      const int hi = selfc ? lo : kc - NP * N;
       float2 v[R1];
       if (act && t < R2) {
 #pragma unroll
@@ -776,8 +779,8 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
 #pragma unroll
         for (int k1 = 0; k1 < R1; ++k1) {
           const int sl = k1 * R2 + t;
-          const int64_t b = (k1 * R2 + R2 - 1 < NP) ? lo : ((k1 * R2 >= NP) ? hi : (sl < NP ? lo : hi));
-          Z[b + (int64_t)sl * st] = (k1 == 0) ? v[0] : cmul(v[k1], twid<-1>(tw, t * k1));
+          const int b = (k1 * R2 + R2 - 1 < NP) ? lo : ((k1 * R2 >= NP) ? hi : (sl < NP ? lo : hi));
+          Z[b + sl * st] = (k1 == 0) ? v[0] : cmul(v[k1], twid<-1>(tw, t * k1));
         }
       }
       __syncthreads();
@@ -785,15 +788,15 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
         float2 w[R2];
         const int s0 = t * R2;
         const bool whole = (s0 + R2 - 1 < NP) || (s0 >= NP);  // R1 even: always
-        const int64_t b = (s0 < NP) ? lo : hi;
+        const int b = (s0 < NP) ? lo : hi;
 #pragma unroll
         for (int n2 = 0; n2 < R2; ++n2) {
           const int sl = s0 + n2;
-          w[n2] = Z[(whole ? b : (sl < NP ? lo : hi)) + (int64_t)sl * st];
+          w[n2] = Z[(whole ? b : (sl < NP ? lo : hi)) + sl * st];
         }
         DFT<R2, N, -1>::run(w);
 #pragma unroll
-        for (int k2 = 0; k2 < R2; ++k2) cp[(int64_t)(t + R1 * k2) * pc + kx] = w[k2];
+        for (int k2 = 0; k2 < R2; ++k2) cp[(t + R1 * k2) * PC + kx] = w[k2];
       }
     }
   }
@@ -803,9 +806,9 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
 // with 0, N): at N = 48 that leaves out two fifths of the pass.
 template <int N, int R1, int R2>
 __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, R1, R2>::MINB) k_fyx3_c2r(const float2* __restrict__ c, float* __restrict__ r,
-                                                               const float2* __restrict__ gtw, float inv,
-                                                               int pc, int pf, int64_t plc, int64_t plf, int lo, int hi) {
-  constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1;
+                                                               const float2* __restrict__ gtw, float inv, int64_t plc,
+                                                               int64_t plf, int lo, int hi) {
+  constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1, PC = plane_pc(N);
   static_assert(T <= 16, "two sequences per warp");
   extern __shared__ float2 sm[];
   float2* tw = sm;
@@ -825,7 +828,7 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
       if (act && t < R2) {
         float2 v[R1];
 #pragma unroll
-        for (int n1 = 0; n1 < R1; ++n1) v[n1] = cp[(int64_t)(R2 * n1 + t) * pc + kx];
+        for (int n1 = 0; n1 < R1; ++n1) v[n1] = cp[(R2 * n1 + t) * PC + kx];
         DFT<R1, N, +1>::run(v);
 #pragma unroll
         for (int k1 = 0; k1 < R1; ++k1) Hc[(k1 * R2 + t) * NH] = (k1 == 0) ? v[0] : cmul(v[k1], twid<+1>(tw, t * k1));
@@ -889,8 +892,8 @@ __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, 
 #pragma unroll
         for (int k2 = 0; k2 < R2; ++k2) {
           const int x = t + R1 * k2;
-          rp[(2 * p) * pf + x] = __fmul_rn(w[k2].x, inv);
-          rp[(2 * p + 1) * pf + x] = __fmul_rn(w[k2].y, inv);
+          rp[(2 * p) * N + x] = __fmul_rn(w[k2].x, inv);
+          rp[(2 * p + 1) * N + x] = __fmul_rn(w[k2].y, inv);
         }
       }
       __syncwarp();

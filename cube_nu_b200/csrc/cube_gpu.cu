@@ -515,16 +515,16 @@ void fft2_run(cube_ctx* c, int64_t nbox, const void* real_in, bool fixed, float 
       return;
     }
   }
-  const int S = std::max(1, 256 / T);
-  const size_t smx = (size_t)(N + S * N) * sizeof(float2);
-  const unsigned gx = (unsigned)((nrows + 2 * S - 1) / (2 * S));
+  using FX = f2::FxShape<N, R1, R2>;
+  const size_t smx = FX::SMEM;
+  const unsigned gx = (unsigned)((nrows + 2 * FX::S - 1) / (2 * FX::S));
   if (fixed) {
     smem_optin(f2::k_fx_r2c<N, R1, R2, long long>, smx);
-    LAUNCH(c, kx, 1, f2::k_fx_r2c<N, R1, R2, long long><<<gx, S * T, smx, c->s>>>((const long long*)real_in, ck, nrows,
+    LAUNCH(c, kx, 1, f2::k_fx_r2c<N, R1, R2, long long><<<gx, f2::FX_T, smx, c->s>>>((const long long*)real_in, ck, nrows,
                                                                                  tw, scale, pt.pr, pt.pc));
   } else {
     smem_optin(f2::k_fx_r2c<N, R1, R2, float>, smx);
-    LAUNCH(c, kx, 1, f2::k_fx_r2c<N, R1, R2, float><<<gx, S * T, smx, c->s>>>((const float*)real_in, ck, nrows, tw,
+    LAUNCH(c, kx, 1, f2::k_fx_r2c<N, R1, R2, float><<<gx, f2::FX_T, smx, c->s>>>((const float*)real_in, ck, nrows, tw,
                                                                              scale, pt.pr, pt.pc));
   }
   smem_optin(f2::k_fcol3<N, R1, R2, 1, 0>, smc);
@@ -533,7 +533,7 @@ void fft2_run(cube_ctx* c, int64_t nbox, const void* real_in, bool fixed, float 
   LAUNCH(c, ky, 1, f2::k_fcol3<N, R1, R2, 1, 0><<<gc, W * T, smc, c->s>>>(ck, tw, W, pt.pc, pt.plc));
   fz_green<N, R1, R2>(c, nbox, ck, green, tw, pt, kz);
   LAUNCH(c, ky, 1, f2::k_fcol3<N, R1, R2, 1, 1><<<gc, W * T, smc, c->s>>>(ck, tw, W, pt.pc, pt.plc));
-  LAUNCH(c, kc, 1, f2::k_fx_c2r<N, R1, R2><<<gx, S * T, smx, c->s>>>(ck, phi_out, nrows, tw, inv, pt.pc, pt.pf));
+  LAUNCH(c, kc, 1, f2::k_fx_c2r<N, R1, R2><<<gx, f2::FX_T, smx, c->s>>>(ck, phi_out, nrows, tw, inv, pt.pc, pt.pf));
 }
 
 bool fft2_size(int n) {
@@ -594,12 +594,12 @@ void fft2_forward(cube_ctx* c, float* real, const Pitch& pt, int cls) {
       return;
     }
   }
-  const int S = std::max(1, 256 / T);
-  const size_t smx = (size_t)(N + S * N) * sizeof(float2);
-  const unsigned gx = (unsigned)((nrows + 2 * S - 1) / (2 * S));
+  using FX = f2::FxShape<N, R1, R2>;
+  const size_t smx = FX::SMEM;
+  const unsigned gx = (unsigned)((nrows + 2 * FX::S - 1) / (2 * FX::S));
   smem_optin(f2::k_fx_r2c<N, R1, R2, float>, smx);
   smem_optin(f2::k_fcol3<N, R1, R2, 1, 0>, smc);
-  LAUNCH(c, cls, 1, f2::k_fx_r2c<N, R1, R2, float><<<gx, S * T, smx, c->s>>>(real, ck, nrows, tw, 1.f, pt.pr, pt.pc));
+  LAUNCH(c, cls, 1, f2::k_fx_r2c<N, R1, R2, float><<<gx, f2::FX_T, smx, c->s>>>(real, ck, nrows, tw, 1.f, pt.pr, pt.pc));
   LAUNCH(c, cls, 1, f2::k_fcol3<N, R1, R2, 1, 0><<<gc, W * T, smc, c->s>>>(ck, tw, W, pt.pc, pt.plc));
   LAUNCH(c, cls, 1, f2::k_fcol3<N, R1, R2, 2, 0><<<gc, W * T, smc, c->s>>>(ck, tw, W, pt.pc, pt.plc));
 }

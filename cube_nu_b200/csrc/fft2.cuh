@@ -168,60 +168,19 @@ struct DFT<4, N, DIR> {
   }
 };
 
-// Two-pass sequence transform over shared memory; element e at base[e*se].
-template <int N, int R1, int R2, int DIR>
-struct Seq {
-  static_assert(R1 * R2 == N, "bad factorisation");
-  __device__ __forceinline__ static void step1(float2* base, int se, int t, const float2* tw) {
-    float2 v[R1];
-#pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1) v[n1] = base[(R2 * n1 + t) * se];
-    DFT<R1, N, DIR>::run(v);
-#pragma unroll
-    for (int k1 = 0; k1 < R1; ++k1) base[(R2 * k1 + t) * se] = (k1 == 0) ? v[0] : cmul(v[k1], twid<DIR>(tw, t * k1));
-  }
-  __device__ __forceinline__ static void step2_load(const float2* base, int se, int t, float2* w, const float2* tw) {
-#pragma unroll
-    for (int n2 = 0; n2 < R2; ++n2) w[n2] = base[(R2 * t + n2) * se];
-    DFT<R2, N, DIR>::run(w);
-  }
-  __device__ __forceinline__ static void step2_store(float2* base, int se, int t, const float2* w) {
-#pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) base[(t + R1 * k2) * se] = w[k2];
-  }
-};
-
 template <int R1, int R2>
 struct TPS {
   static constexpr int T = R1 > R2 ? R1 : R2;  // threads per sequence
 };
 
-// Full in-place transform of the sequences handled by this thread group.
-// Thread (s, t): s = sequence slot, t in [0, T).  All threads of the block call it.
-template <int N, int R1, int R2, int DIR>
-__device__ __forceinline__ void seq_transform(float2* base, int se, int t, const float2* tw) {
-  using S = Seq<N, R1, R2, DIR>;
-  if (t < R2) S::step1(base, se, t, tw);
-  __syncthreads();
-  float2 w[R2];
-  if (t < R1) S::step2_load(base, se, t, w, tw);
-  __syncthreads();
-  if (t < R1) S::step2_store(base, se, t, w);
-  __syncthreads();
-}
-
-// Same as seq_transform, for thread groups where some threads have no sequence this
-// round (they still take part in the barriers).
-template <int N, int R1, int R2, int DIR>
-__device__ __forceinline__ void seq_transform_g(float2* base, int se, int t, const float2* tw, bool active) {
-  using S = Seq<N, R1, R2, DIR>;
-  if (active && t < R2) S::step1(base, se, t, tw);
-  __syncthreads();
-  float2 w[R2];
-  if (active && t < R1) S::step2_load(base, se, t, w, tw);
-  __syncthreads();
-  if (active && t < R1) S::step2_store(base, se, t, w);
-  __syncthreads();
+// Slot of (k1, n2) in the exchange between the two steps, skewed so that neither the writes
+// (fixed k1) nor the reads (fixed n2) meet on a bank.
+template <int R1, int R2>
+__device__ __forceinline__ int skew(int k1, int n2) {
+  int j = n2 + k1;  // < R1 + R2
+  if (R1 <= R2) j = (j >= R2) ? j - R2 : j;
+  else j = j % R2;
+  return k1 * R2 + j;
 }
 
 // Mesh layouts (both in place, potential written over the input):
@@ -233,41 +192,75 @@ __device__ __forceinline__ void seq_transform_g(float2* base, int se, int t, con
 // in the same units (plr, plc, plf).
 
 // ---------------------------------------------------------------------------------
-// X pass, r2c.  Block: S packed sequences (2S real rows); blockDim = S*T.  In place:
-// the block loads all its rows before writing their spectra.
+// X pass, r2c.  Block: S = 256/T packed sequences (2S real rows), T threads side by side each.
+// A thread loads its R1 points of both rows straight from memory, and the exchange between
+// the steps is skewed; staging the rows in shared memory first, with an exchange that read
+// it at a stride of R2, cost 0.98 and 1.12 ms in 20 transforms of a 256^3 mesh each way, 0.52
+// and 0.49 now.  In place: a sequence's rows are loaded before the first barrier.
 // ---------------------------------------------------------------------------------
+constexpr int FX_T = 256;
+template <int N, int R1, int R2>
+struct FxShape {
+  static constexpr int T = TPS<R1, R2>::T, S = FX_T / T, MINB = T <= 18 ? 3 : 2;
+  static constexpr size_t SMEM = (size_t)(N + S * N) * 8;
+};
+
 template <int N, int R1, int R2, typename IN>
-__global__ void __launch_bounds__(256) k_fx_r2c(const IN* r, float2* c, int64_t nrows, const float2* __restrict__ gtw,
-                                                float scale, int pr, int pc) {
-  constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1;
+__global__ void __launch_bounds__(FX_T, FxShape<N, R1, R2>::MINB) k_fx_r2c(const IN* r, float2* c, int64_t nrows,
+                                                                         const float2* __restrict__ gtw, float scale,
+                                                                         int pr, int pc) {
+  using FX = FxShape<N, R1, R2>;
+  constexpr int T = FX::T, NH = N / 2 + 1;
   extern __shared__ float2 sm[];
   float2* tw = sm;
-  float2* Z = sm + N;
-  const int S = blockDim.x / T;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = gtw[i];
-  const int64_t row0 = (int64_t)blockIdx.x * 2 * S;
-  const int nr = (int)min((int64_t)2 * S, nrows - row0);
-  for (int i = threadIdx.x; i < 2 * S * N; i += blockDim.x) {
-    const int row = i / N, x = i - row * N;
-    float f = 0.f;
-    if (row < nr) {
-      const IN v = r[(row0 + row) * pr + x];
-      if (sizeof(IN) == 8) f = (float)((double)(long long)v * 9.094947017729282e-13);  // 2^-40
-      else f = (float)v;
-      f = __fmul_rn(f, scale);
+  for (int i = threadIdx.x; i < N; i += FX_T) tw[i] = gtw[i];
+  const int s = threadIdx.x / T, t = threadIdx.x % T;
+  const int64_t row = ((int64_t)blockIdx.x * FX::S + s) * 2;
+  const bool act = s < FX::S && row < nrows, two = row + 1 < nrows;
+  float2* Zr = sm + N + (s < FX::S ? s : 0) * N;
+  float2 v[R1];
+  if (act && t < R2) {
+    const IN* a = r + row * pr + t;
+    const IN* b = a + (two ? pr : 0);
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1) {
+      float fa, fb;
+      if (sizeof(IN) == 8) {
+        fa = (float)((double)(long long)a[R2 * n1] * 9.094947017729282e-13);  // 2^-40
+        fb = (float)((double)(long long)b[R2 * n1] * 9.094947017729282e-13);
+      } else {
+        fa = (float)a[R2 * n1];
+        fb = (float)b[R2 * n1];
+      }
+      v[n1] = make_float2(__fmul_rn(fa, scale), __fmul_rn(two ? fb : 0.f, scale));
     }
-    reinterpret_cast<float*>(Z + (row >> 1) * N + x)[row & 1] = f;
+  }
+  __syncthreads();  // the table
+  if (act && t < R2) {
+    DFT<R1, N, -1>::run(v);
+#pragma unroll
+    for (int k1 = 0; k1 < R1; ++k1) Zr[skew<R1, R2>(k1, t)] = (k1 == 0) ? v[0] : cmul(v[k1], twid<-1>(tw, t * k1));
   }
   __syncthreads();
-  const int s = threadIdx.x / T, t = threadIdx.x - s * T;
-  seq_transform<N, R1, R2, -1>(Z + s * N, 1, t, tw);
-  for (int i = threadIdx.x; i < S * NH; i += blockDim.x) {
-    const int q = i / NH, k = i - q * NH;
-    if (2 * q >= nr) continue;
-    const float2 z = Z[q * N + k];
-    const float2 zc = Z[q * N + ((N - k) % N)];
-    c[(row0 + 2 * q) * pc + k] = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
-    if (2 * q + 1 < nr) c[(row0 + 2 * q + 1) * pc + k] = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
+  float2 w[R2];
+  if (act && t < R1) {
+#pragma unroll
+    for (int n2 = 0; n2 < R2; ++n2) w[n2] = Zr[skew<R1, R2>(t, n2)];
+    DFT<R2, N, -1>::run(w);
+  }
+  __syncthreads();
+  if (act && t < R1) {
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) Zr[t + R1 * k2] = w[k2];
+  }
+  __syncthreads();
+  if (act) {
+    float2* c0 = c + row * pc;
+    for (int k = t; k < NH; k += T) {
+      const float2 z = Zr[k], zc = Zr[k == 0 ? 0 : N - k];
+      c0[k] = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
+      if (two) c0[pc + k] = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
+    }
   }
 }
 
@@ -610,38 +603,60 @@ __host__ inline void fz_stream_shape(int N, int T, int& W, int& ncg) {
 __host__ inline size_t fz_stream_smem(int N, int W) { return (size_t)N * 8 + (size_t)2 * N * W * 12; }
 
 // ---------------------------------------------------------------------------------
-// X' pass, c2r, divided `reps` times by `norm`.  In place (complex rows pc -> real rows pf).
+// X' pass, c2r, times `inv`: the mirror image of k_fx_r2c.  In place (complex rows pc -> real
+// rows pf).
 // ---------------------------------------------------------------------------------
 template <int N, int R1, int R2>
-__global__ void __launch_bounds__(256) k_fx_c2r(const float2* c, float* r, int64_t nrows, const float2* __restrict__ gtw,
-                                                float inv, int pc, int pf) {
-  constexpr int T = TPS<R1, R2>::T, NH = N / 2 + 1;
+__global__ void __launch_bounds__(FX_T, FxShape<N, R1, R2>::MINB) k_fx_c2r(const float2* c, float* r, int64_t nrows,
+                                                                         const float2* __restrict__ gtw, float inv, int pc,
+                                                                         int pf) {
+  using FX = FxShape<N, R1, R2>;
+  constexpr int T = FX::T, NH = N / 2 + 1;
   extern __shared__ float2 sm[];
   float2* tw = sm;
-  float2* Z = sm + N;
-  const int S = blockDim.x / T;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = gtw[i];
-  const int64_t row0 = (int64_t)blockIdx.x * 2 * S;
-  const int nr = (int)min((int64_t)2 * S, nrows - row0);
-  for (int i = threadIdx.x; i < S * N; i += blockDim.x) {
-    const int q = i / N, x = i - q * N;
-    float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
-    const int k = (x < NH) ? x : N - x;
-    if (2 * q < nr) a0 = c[(row0 + 2 * q) * pc + k];
-    if (2 * q + 1 < nr) a1 = c[(row0 + 2 * q + 1) * pc + k];
-    if (k == 0 || 2 * k == N) { a0.y = 0.f; a1.y = 0.f; }
-    if (x >= NH) { a0.y = -a0.y; a1.y = -a1.y; }
-    Z[q * N + x] = make_float2(a0.x - a1.y, a0.y + a1.x);
+  for (int i = threadIdx.x; i < N; i += FX_T) tw[i] = gtw[i];
+  const int s = threadIdx.x / T, t = threadIdx.x % T;
+  const int64_t row = ((int64_t)blockIdx.x * FX::S + s) * 2;
+  const bool act = s < FX::S && row < nrows, two = row + 1 < nrows;
+  float2* Zr = sm + N + (s < FX::S ? s : 0) * N;
+  float2 v[R1];
+  if (act && t < R2) {
+    const float2* c0 = c + row * pc;
+    const float2* c1 = c0 + (two ? pc : 0);
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1) {  // the Hermitian extension of both rows, packed
+      const int x = R2 * n1 + t, k = x < NH ? x : N - x;
+      float2 a0 = c0[k], a1 = c1[k];
+      if (!two) a1 = make_float2(0.f, 0.f);
+      if (k == 0 || 2 * k == N) {
+        a0.y = 0.f;
+        a1.y = 0.f;
+      }
+      if (x >= NH) {
+        a0.y = -a0.y;
+        a1.y = -a1.y;
+      }
+      v[n1] = make_float2(a0.x - a1.y, a0.y + a1.x);
+    }
+  }
+  __syncthreads();  // the table, and every row is read
+  if (act && t < R2) {
+    DFT<R1, N, +1>::run(v);
+#pragma unroll
+    for (int k1 = 0; k1 < R1; ++k1) Zr[skew<R1, R2>(k1, t)] = (k1 == 0) ? v[0] : cmul(v[k1], twid<+1>(tw, t * k1));
   }
   __syncthreads();
-  const int s = threadIdx.x / T, t = threadIdx.x - s * T;
-  seq_transform<N, R1, R2, +1>(Z + s * N, 1, t, tw);
-  for (int i = threadIdx.x; i < 2 * S * N; i += blockDim.x) {
-    const int row = i / N, x = i - row * N;
-    if (row >= nr) continue;
-    const float2 z = Z[(row >> 1) * N + x];
-    float v = (row & 1) ? z.y : z.x;
-    r[(row0 + row) * pf + x] = __fmul_rn(v, inv);
+  if (act && t < R1) {
+    float2 w[R2];
+#pragma unroll
+    for (int n2 = 0; n2 < R2; ++n2) w[n2] = Zr[skew<R1, R2>(t, n2)];
+    DFT<R2, N, +1>::run(w);
+    float* r0 = r + row * pf + t;
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) {
+      r0[R1 * k2] = __fmul_rn(w[k2].x, inv);
+      if (two) r0[pf + R1 * k2] = __fmul_rn(w[k2].y, inv);
+    }
   }
 }
 
@@ -678,14 +693,6 @@ struct Plane3Sm {
   // inverse: half spectrum H[N][NH]
   static constexpr size_t INV = (size_t)(N + N * NH) * 8;
 };
-
-template <int R1, int R2>
-__device__ __forceinline__ int skew(int k1, int n2) {
-  int j = n2 + k1;  // < R1 + R2
-  if (R1 <= R2) j = (j >= R2) ? j - R2 : j;
-  else j = j % R2;
-  return k1 * R2 + j;
-}
 
 template <int N, int R1, int R2, typename IN>
 __global__ void __launch_bounds__(PlaneShape<N, R1, R2>::THREADS, PlaneShape<N, R1, R2>::MINB) k_fxy3_r2c(const IN* __restrict__ r, float2* __restrict__ c,

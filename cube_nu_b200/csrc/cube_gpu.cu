@@ -3073,12 +3073,17 @@ struct cube_dpm {
 
 namespace {
 
+void dpm_deposit(cube_dpm* d, int64_t np, const float* x, float* rho, int pr, int64_t pl) {
+  auto k = dpm_pairs(d->n, rho, pr, pl) ? k_dpm_deposit<true> : k_dpm_deposit<false>;
+  k<<<nblk(np), 256, 0, d->c->s>>>(d->n, np, x, d->mass, rho, pr, pl);
+}
+
 // Force mesh Fm = grad_h Gconv(rho) of the particles at x.
 int dpm_force_mesh(cube_dpm* d, const float* x, int64_t np) {
   cube_ctx* c = d->c;
   const int n = d->n;
   CK(cudaMemsetAsync(d->mesh, 0, mesh_bytes(c, n, 1, false), c->s));
-  if (np > 0) k_dpm_deposit<<<nblk(np), 256, 0, c->s>>>(n, np, x, d->mass, d->mesh, d->pt.pr, d->pt.plr);
+  if (np > 0) dpm_deposit(d, np, x, d->mesh, d->pt.pr, d->pt.plr);
   launch_fft(c, n, 1, d->mesh, false, 1.f, d->mesh, reinterpret_cast<float2*>(d->mesh), c->green1, (float)n, 3, 1);
   k_force_pm1<<<force_grid(n), FORCE_T, 0, c->s>>>(n, d->mesh, d->pt.pf, d->pt.plf, d->fm);
   c->launches += 7;
@@ -3151,7 +3156,7 @@ int cube_dpm_density(cube_dpm* d, const float* x, int64_t np, float* rho) {
   CK(cudaSetDevice(d->c->device));
   const int n = d->n;
   CK(cudaMemsetAsync(rho, 0, (size_t)n * n * n * 4, d->c->s));
-  if (np > 0) k_dpm_deposit<<<nblk(np), 256, 0, d->c->s>>>(n, np, x, d->mass, rho, n, (int64_t)n * n);
+  if (np > 0) dpm_deposit(d, np, x, rho, n, (int64_t)n * n);
   ++d->c->launches;
   return dpm_finish(d);
 }

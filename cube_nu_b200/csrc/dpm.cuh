@@ -43,7 +43,11 @@ __device__ __forceinline__ void dpm_cells(int fl, int n, int c[3]) {
   c[2] = wrap1(f + 1, n);
 }
 
-// rho += m * W, into a mesh with row pitch pr and plane pitch pl (floats).
+// rho += m * W, into a mesh with row pitch pr and plane pitch pl (floats).  Bound by the L2
+// reductions.  PAIR (dpm_pairs): the three cells of a row are two 8-byte reductions of aligned
+// cells, the fourth value zero, instead of three of 4 bytes: 18 a particle for 27 (0.100 ms for
+// 2^21 particles on 256^3 cells, 0.132 one by one).  A row that wraps has its cells one by one.
+template <bool PAIR>
 __global__ void k_dpm_deposit(int n, int64_t np, const float* __restrict__ x, float m, float* __restrict__ rho, int pr,
                               int64_t pl) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -52,16 +56,31 @@ __global__ void k_dpm_deposit(int n, int64_t np, const float* __restrict__ x, fl
   int f[3][3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) dpm_cells(dpm_w(x[3 * i + d], w[d], dw), n, f[d]);
+  const bool wraps = f[0][2] != f[0][0] + 2, odd = f[0][0] & 1;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const int64_t z = (int64_t)f[2][c] * pl;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       const int64_t y = (int64_t)f[1][b] * pr;
+      float v[3];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) atomicAdd(&rho[z + y + f[0][a]], m * w[0][a] * w[1][b] * w[2][c]);
+      for (int a = 0; a < 3; ++a) v[a] = m * w[0][a] * w[1][b] * w[2][c];
+      if (PAIR && !wraps) {  // n even: the pairs end at cell n - 1 at most
+        float2* const p = reinterpret_cast<float2*>(&rho[z + y + (f[0][0] & ~1)]);
+        atomicAdd(p, odd ? make_float2(0.f, v[0]) : make_float2(v[0], v[1]));
+        atomicAdd(p + 1, odd ? make_float2(v[1], v[2]) : make_float2(v[2], 0.f));
+      } else {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) atomicAdd(&rho[z + y + f[0][a]], v[a]);
+      }
     }
   }
+}
+
+// Cells 2k and 2k+1 of every row are one aligned 8-byte word.
+inline bool dpm_pairs(int n, const float* rho, int pr, int64_t pl) {
+  return n % 2 == 0 && pr % 2 == 0 && pl % 2 == 0 && (reinterpret_cast<uintptr_t>(rho) & 7) == 0;
 }
 
 // F_i = sum_c W Fm(c) (Fm: float4 per cell, dense, x fastest); then the KDK kick

@@ -1451,7 +1451,8 @@ static int enqueue_kick_a(cube_ctx* c) {
     const int64_t n3 = (int64_t)n * n * n;
     if (foff + (size_t)n3 * sizeof(float4) <= c->arena_bytes) {
       float4* force = reinterpret_cast<float4*>(reinterpret_cast<char*>(c->arena) + foff);
-      LAUNCH(c, K_INT_PM1, 1, k_force_pm1<<<force_grid(n), FORCE_T, 0, c->s>>>(n, phi, m.pt.pf, m.pt.plf, force));
+      auto kf = force_deep(n) ? k_force_pm1<FORCE_Z> : k_force_pm1<1>;
+      LAUNCH(c, K_INT_PM1, 1, kf<<<force_grid(n, force_deep(n) ? FORCE_Z : 1), FORCE_T, 0, c->s>>>(n, phi, m.pt.pf, m.pt.plf, force));
       LAUNCH(c, K_INT_PM1, 1, k_interp_pm1_force<<<nblk(npo), 256, 0, c->s>>>(G, npo, xpo, pco, force, vpo, c->sd));
     } else {
       LAUNCH(c, K_INT_PM1, 1, k_interp_pm1<<<nblk(npo), 256, 0, c->s>>>(G, npo, xpo, pco, phi, vpo, c->sd, m.pt.pf, m.pt.plf));
@@ -3085,7 +3086,8 @@ int dpm_force_mesh(cube_dpm* d, const float* x, int64_t np) {
   CK(cudaMemsetAsync(d->mesh, 0, mesh_bytes(c, n, 1, false), c->s));
   if (np > 0) dpm_deposit(d, np, x, d->mesh, d->pt.pr, d->pt.plr);
   launch_fft(c, n, 1, d->mesh, false, 1.f, d->mesh, reinterpret_cast<float2*>(d->mesh), c->green1, (float)n, 3, 1);
-  k_force_pm1<<<force_grid(n), FORCE_T, 0, c->s>>>(n, d->mesh, d->pt.pf, d->pt.plf, d->fm);
+  auto kf = force_deep(n) ? k_force_pm1<FORCE_Z> : k_force_pm1<1>;
+  kf<<<force_grid(n, force_deep(n) ? FORCE_Z : 1), FORCE_T, 0, c->s>>>(n, d->mesh, d->pt.pf, d->pt.plf, d->fm);
   c->launches += 7;
   return 0;
 }

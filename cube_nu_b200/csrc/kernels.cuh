@@ -1437,22 +1437,43 @@ __global__ void k_interp_pm1(Geo G, int64_t np, const void* __restrict__ xp, con
 // (particle_mesh.f90:224-247): at every coarse cell j (0-based, periodic) the three
 // components grad4(phi(j-2), phi(j-1), phi(j+1), phi(j+2)), with the same FP32
 // operations as tsc_gather_force, stored as float4 (fx, fy, fz, 0), x fastest.
-// Grid (blocks along x, y, z) of FORCE_T cells along x: with a flat index and 64-bit divisions
-// it took 0.24 ms at 256^3, five times the write of the force mesh.
-constexpr int FORCE_T = 128;
-inline dim3 force_grid(int nc) { return dim3((unsigned)((nc + FORCE_T - 1) / FORCE_T), (unsigned)nc, (unsigned)nc); }
+// Grid (blocks along x, y, z): FORCE_T cells along x and, per thread, ZS along z.  Bound by the
+// write of 16 bytes a cell; with one cell a thread the blocks of a large mesh come and go too
+// fast to keep enough loads in flight: 0.119 ms at 256^3 cells, 0.090 with four (the write and
+// the read of phi alone: 0.050).  A mesh whose blocks of four cells are fewer than two rounds
+// of the chip's (2 x 16 x 148) keeps one (64^3: 4.0 us against 4.5).
+constexpr int FORCE_T = 128, FORCE_Z = 4;
+inline dim3 force_grid(int nc, int zs = 1) {
+  return dim3((unsigned)((nc + FORCE_T - 1) / FORCE_T), (unsigned)nc, (unsigned)((nc + zs - 1) / zs));
+}
+inline bool force_deep(int nc) {
+  const dim3 g = force_grid(nc, FORCE_Z);
+  return (int64_t)g.x * g.y * g.z >= 2 * 16 * 148;
+}
+template <int ZS>
 __global__ void __launch_bounds__(FORCE_T) k_force_pm1(int nc, const float* __restrict__ phi, int pf, int64_t pl,
                                                        float4* __restrict__ force) {
-  const int x = blockIdx.x * FORCE_T + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
+  const int x = blockIdx.x * FORCE_T + threadIdx.x, y = blockIdx.y, z0 = blockIdx.z * ZS;
   if (x >= nc) return;
-  const float* row = phi + (int64_t)z * pl + (int64_t)y * pf;
-  const float* col = phi + (int64_t)z * pl + x;
-  const float* line = phi + (int64_t)y * pf + x;
-  auto X = [&](int d) { return __ldg(row + wrap1(x + d, nc)); };
-  auto Y = [&](int d) { return __ldg(col + (int64_t)wrap1(y + d, nc) * pf); };
-  auto Z = [&](int d) { return __ldg(line + (int64_t)wrap1(z + d, nc) * pl); };
-  force[((int64_t)z * nc + y) * nc + x] = make_float4(grad4(X(-2), X(-1), X(1), X(2)), grad4(Y(-2), Y(-1), Y(1), Y(2)),
-                                                      grad4(Z(-2), Z(-1), Z(1), Z(2)), 0.f);
+  const int xm2 = wrap1(x - 2, nc), xm1 = wrap1(x - 1, nc), xp1 = wrap1(x + 1, nc), xp2 = wrap1(x + 2, nc);
+  const float* const row = phi + (int64_t)y * pf;
+  const float* const ym2 = phi + (int64_t)wrap1(y - 2, nc) * pf + x;
+  const float* const ym1 = phi + (int64_t)wrap1(y - 1, nc) * pf + x;
+  const float* const yp1 = phi + (int64_t)wrap1(y + 1, nc) * pf + x;
+  const float* const yp2 = phi + (int64_t)wrap1(y + 2, nc) * pf + x;
+  float line[ZS + 4];  // phi(x, y, z0 - 2 ..)
+#pragma unroll
+  for (int k = 0; k < ZS + 4; ++k) line[k] = __ldg(row + x + (int64_t)wrapi(z0 - 2 + k, nc) * pl);
+#pragma unroll
+  for (int k = 0; k < ZS; ++k) {
+    const int z = z0 + k;
+    if (z >= nc) break;
+    const int64_t o = (int64_t)z * pl;
+    force[((int64_t)z * nc + y) * nc + x] =
+        make_float4(grad4(__ldg(row + o + xm2), __ldg(row + o + xm1), __ldg(row + o + xp1), __ldg(row + o + xp2)),
+                    grad4(__ldg(ym2 + o), __ldg(ym1 + o), __ldg(yp1 + o), __ldg(yp2 + o)),
+                    grad4(line[k], line[k + 1], line[k + 3], line[k + 4]), 0.f);
+  }
 }
 
 // PM1 interpolation + kick from the force mesh: the 27 TSC points of a particle are the

@@ -151,15 +151,14 @@ class Clocks:
 def kernel_bytes(p, name: str, n_particles: int, napm, fixed: bool):
     """Algorithmic HBM bytes a kernel class must move over one whole step (all its
     launches together): mesh passes read and write each cell once at the element size
-    of the pass, particle kernels read each particle's code and velocity once, the
-    deposit adds 27 read-modify-writes per particle and box it lands in."""
+    of the pass, particle kernels read each particle's code and velocity once, the PM1
+    deposit adds 27 read-modify-writes per particle."""
     bx = 3 * p.izipx
-    rb = 8 if fixed else 4
 
-    def mesh(n, nbox, what, rb=rb):
+    def mesh(n, nbox, what):  # PM2 and PM3 meshes are float in both deposit forms
         n3 = n ** 3 * nbox
         nh = n * n * (n // 2 + 1) * nbox
-        return {"x": n3 * rb + nh * 8, "y": 2 * nh * 8, "z": 2 * nh * 8 + n * n * (n // 2 + 1) * 4,
+        return {"x": n3 * 4 + nh * 8, "y": 2 * nh * 8, "z": 2 * nh * 8 + n * n * (n // 2 + 1) * 4,
                 "c": nh * 8 + n3 * 4}[what]
 
     if name.startswith("fft_") and name.endswith("_pm3"):
@@ -167,21 +166,23 @@ def kernel_bytes(p, name: str, n_particles: int, napm, fixed: bool):
         n = p.nft(2)
         nb = int(napm[2]) if napm is not None else p.ns3
         what = {"fft_x_pm3": "x", "fft_y_pm3": "y", "fft_z_green_pm3": "z", "fft_c2r_pm3": "c"}[name]
-        # the PM3 mesh is float in both deposit forms (the owner-computes fixed-point
-        # deposit writes the converted sums)
-        return mesh(n, nb, what, rb=4) * (2 if what == "y" else 1)
+        # whole boxes, though the inverse passes leave out the planes of the potential that
+        # no force reads (10 of a 144^3 box's 144)
+        return mesh(n, nb, what) * (2 if what == "y" else 1)
     if name.startswith("fft_") and name.endswith("_pm2"):
         what = {"fft_x_pm2": "x", "fft_y_pm2": "y", "fft_z_green_pm2": "z", "fft_c2r_pm2": "c"}[name]
         return mesh(p.ngt, p.ntiles, what) * (2 if what == "y" else 1)
-    if name == "deposit_pm3" and fixed:
-        # owner-computes form: every cell of every box written once as float (no memset,
-        # no read-back), each particle's position code read once
+    # PM2 and PM3 deposits, owner-computes: every cell of every box written once as float
+    # (no memset, no read-back), each particle's position code read once (PM2: once per tile
+    # whose ghost region holds it)
+    if name == "deposit_pm2":
+        return int(p.ntiles * p.ngt ** 3 * 4 + n_particles * (1 + 2 * p.ncb / p.nt) ** 3 * bx)
+    if name == "deposit_pm3":
         nbs = napm if napm is not None else [0, 0, p.ns3, 0, 0, 0]
         return int(sum(int(nbs[c]) * p.nft(c) ** 3 * 4 for c in range(2, 6)) + n_particles * bx)
-    if name in ("deposit_pm1", "deposit_pm2", "deposit_pm3"):
+    if name == "deposit_pm1":
         # read position code + cell index per particle, one read-modify-write of 27 cells
-        boxes = {"deposit_pm1": 1.0, "deposit_pm2": (1 + 2 * p.ncb / p.nt) ** 3, "deposit_pm3": (1 + 2 / p.ntt) ** 3}[name]
-        return int(n_particles * (bx + 4 + boxes * 27 * 2 * rb))
+        return int(n_particles * (bx + 4 + 27 * 2 * (8 if fixed else 4)))
     if name in ("interp_pm1", "interp_pm2", "interp_pm3"):
         # position code + cell, velocity read+write, 27 force points x 3 (from phi)
         return int(n_particles * (bx + 4 + 24 + 27 * 4))

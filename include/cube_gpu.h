@@ -51,8 +51,8 @@ extern "C" {
 #define CUBE_DEVERR_FIXED_OVERFLOW 0x20u
 
 /* Deposit arithmetic. */
-#define CUBE_DEPOSIT_FP32 0  /* plain form: FP32 atomics (order-dependent rounding)           */
-#define CUBE_DEPOSIT_FIXED 1 /* chosen form: int64 fixed-point atomics (deterministic)         */
+#define CUBE_DEPOSIT_FP32 0  /* plain form: FP32 sums in no fixed order (rounding varies)      */
+#define CUBE_DEPOSIT_FIXED 1 /* chosen form: int64 fixed-point sums (deterministic)            */
 
 /*
  * Run parameters.  Names and meanings follow parameters.f90; derived sizes
@@ -83,7 +83,11 @@ typedef struct cube_params {
                           above 16384: 16384); longer cells take a rank sort in HBM       */
   int32_t step_graph;  /* 1: cube_gpu_step replays each step as one captured CUDA graph   */
   int32_t pp_queue;    /* 1: PP as an autotuned work queue over cells (needs int8 codes, or
-                          int16 with nt < 127); 0: one thread per particle                 */
+                          int16 with nt < 127); 0: one thread per particle, except that once a
+                          cell holds more than 64 particles the cells of more than 16 take
+                          the queue's kernel at a fixed shape (same forces, bit for bit; its
+                          buffers, 4 bytes per particle and 8 per coarse cell, are allocated
+                          then, and without memory for them a thread per particle serves) */
   int32_t nslab;       /* z-slabs the periodic box is split into, one rank each (0 or 1: one
                           rank holds the whole box); nnt must be a multiple of nslab      */
   int32_t slab;        /* this rank's slab: tile layers [slab*L, (slab+1)*L) along z with

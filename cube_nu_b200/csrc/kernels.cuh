@@ -1710,16 +1710,29 @@ __global__ void __launch_bounds__(1024) k_build_lists(const int32_t* __restrict_
 // coarse cells its range can reach; equivalent to the reference's PP-cell lists
 // (the PP cell 4/rsf fine cells is wider than the range 3.5/rsf).
 // =================================================================================
-// F_ra of kick.f90 at r = e * apm / 2 <= apm, from e, apm's coefficient c = (1/35)/apm^2 and
-// 12/e^2 (the S2 cloud's force; 1/r^2 beyond).
+// F_ra of kick.f90 at r = e * apm / 2 <= apm, over apm's coefficient c = (1/35)/apm^2 (the S2
+// cloud's force; 1/r^2 beyond).  The outer branch is the polynomial of kick.f90 written in
+// t = 2 - e, whose terms are of the sum's size: in e they are a hundred times it and their
+// rounding made the force's largest error.
 // Rounded step by step (no contraction), so that every kernel gives the same bits.
-__device__ __forceinline__ float F_s2(float e, float c, float twelve_over_e2) {
-  const float e2 = __fmul_rn(e, e);
-  const float near = __fmul_rn(
-      e, __fmaf_rn(e2, __fmaf_rn(e, __fmaf_rn(e, __fmaf_rn(e, -21.f, 48.f), 70.f), -224.f), 224.f));
-  const float poly = __fmaf_rn(
-      e, __fmaf_rn(e, __fmaf_rn(e, __fmaf_rn(e, __fmaf_rn(e, __fmaf_rn(e, 7.f, -48.f), 70.f), 224.f), -840.f), 896.f), -224.f);
-  return __fmul_rn(c, e > 1.f ? __fadd_rn(poly, twelve_over_e2) : near);
+__device__ __forceinline__ float F_s2_near(float e) {  // e <= 1
+  return __fmul_rn(
+      e, __fmaf_rn(__fmul_rn(e, e), __fmaf_rn(e, __fmaf_rn(e, __fmaf_rn(e, -21.f, 48.f), 70.f), -224.f), 224.f));
+}
+__device__ __forceinline__ float F_s2(float e, float twelve_over_e2) {
+  const float t = __fsub_rn(2.f, e);
+  const float far = __fmaf_rn(
+      t, __fmaf_rn(t, __fmaf_rn(t, __fmaf_rn(t, __fmaf_rn(t, __fmaf_rn(t, 7.f, -36.f), 10.f), 16.f), 24.f), 32.f), 32.f);
+  // the terms in e up to t^6; 12/e^2 is apart
+  return e > 1.f ? __fadd_rn(far, twelve_over_e2) : F_s2_near(e);
+}
+// 1/r^2 less F_s2, over c, for 1 < e: 140/e^2 less the two terms above.  Its terms cancel up to
+// t^4 (140/e^2 - 12/e^2 = 128/e^2 is a power series in t with the same ones), and what is left
+// is a product, with no cancellation.
+__device__ __forceinline__ float F_s2_rest(float e, float one_over_e2) {
+  const float t = __fsub_rn(2.f, e), t2 = __fmul_rn(t, t);
+  return __fmul_rn(__fmul_rn(__fmul_rn(t2, t2), t),
+                   __fmaf_rn(__fmaf_rn(t, -10.f, 24.f), one_over_e2, __fmaf_rn(t, -7.f, 36.f)));
 }
 
 // Candidate coordinate (xq in kick.f90:424): ((lq + (u+0.5)*x_res) * ratio_cs) rounded to
@@ -1739,8 +1752,8 @@ struct PPi {
   float xf[3];
   int l[3], lo[3], hi[3];
   float range, range2;
-  float k_range, c_range, p_range;  // 2/range, (1/35)/range^2, 3 range^2: F_s2 of the range
-  float k_app, c_app, p_app;        // the same of the softening app (k_app infinite: none)
+  float k_range, c_range, p_range;  // 2/range, (1/35)/range^2, range^2/4: F_s2 of the range
+  float k_app, c_app, p_app;        // 2/app, (1/35)/app^2, 3 app^2: of the softening (k_app infinite: none)
   float acc[3];
   unsigned pairs, cand;  // of this particle (item): well below 2^32
 
@@ -1750,7 +1763,7 @@ struct PPi {
     range2 = __fmul_rn(range, range);
     k_range = __fdiv_rn(2.f, range);
     c_range = __fdiv_rn(__fdiv_rn(1.f, 35.f), range2);
-    p_range = 3.f * range2;
+    p_range = 0.25f * range2;
     k_app = G.app > 0.f ? __fdiv_rn(2.f, G.app) : __int_as_float(0x7f800000);
     c_app = G.app > 0.f ? __fdiv_rn(__fdiv_rn(1.f, 35.f), __fmul_rn(G.app, G.app)) : 0.f;
     p_app = 3.f * G.app * G.app;
@@ -1774,16 +1787,24 @@ struct PPi {
   // square root and one Newton step (y + y (1/2 - r2 y^2 / 2)), good to about one unit in the
   // last place; the force law and the projection multiply by it.  With IEEE square root and
   // divisions (up to eight a pair) the law took three times the instructions (with the packed
-  // separations, the heavy-cell PP of 128^3 clustered particles: 24.8 -> 13.4 ms); the force's
-  // error against 64 bits is the same.
+  // separations, the heavy-cell PP of 128^3 clustered particles: 24.8 -> 13.6 ms).  The force
+  // of the outer pairs as a product without cancellation (F_s2_rest) costs 0.5 ms of that again
+  // and takes the velocities' error against 64 bits below the IEEE form's (a kick of three
+  // tiles a side: 3.8e-7, 4.1e-7 before F_s2_rest, 3.1e-7 now).
   __device__ __forceinline__ void accum(float rv0, float rv1, float rv2, float r2) {
     const float y = rsqrtf(r2);
     const float inv = __fmaf_rn(y, __fmaf_rn(__fmul_rn(__fmul_rn(-0.5f, r2), y), y, 0.5f), y);
     const float inv2 = __fmul_rn(inv, inv), r = __fmul_rn(r2, inv);
-    float sc = inv2;
-    const float ea = __fmul_rn(r, k_app);
-    if (ea <= 2.f) sc = F_s2(ea, c_app, __fmul_rn(p_app, inv2));
-    sc = __fsub_rn(sc, F_s2(__fmul_rn(r, k_range), c_range, __fmul_rn(p_range, inv2)));
+    const float ea = __fmul_rn(r, k_app), e = __fmul_rn(r, k_range);
+    float near = inv2, extra = 0.f;
+    if (ea <= 2.f) {
+      near = __fmul_rn(c_app, F_s2(ea, __fmul_rn(p_app, inv2)));
+      extra = __fsub_rn(near, inv2);
+    }
+    // both sides of e = 1, without a branch
+    const float rest = __fmaf_rn(c_range, F_s2_rest(e, __fmul_rn(p_range, inv2)), extra);
+    const float inner = __fmaf_rn(-c_range, F_s2_near(e), near);
+    float sc = e > 1.f ? rest : inner;
     sc = __fmul_rn(sc, inv);
     acc[0] = __fmaf_rn(rv0, sc, acc[0]);
     acc[1] = __fmaf_rn(rv1, sc, acc[1]);

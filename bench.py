@@ -44,14 +44,15 @@ from cube_nu_b200.params import DEPOSIT_FIXED, DEPOSIT_FP32, config_512, config_
 
 METRIC = "particle-steps/s P3M KDK @512^3"
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0}
-# DRAM bytes (read + write) per class-2 PM3 box of 144^3, measured once with ncu on the
-# proxy workload (one launch over 64 boxes) and kept here as constants: the 512^3 launch is
+# DRAM bytes (read + write) per class-2 PM3 box of 144^3, measured once with ncu on one tile
+# of the workload (one launch over 64 boxes) and kept here as constants: the 512^3 launch is
 # too large to capture.  Traffic grows with the number of boxes, so a launch over B such
 # boxes moves B times these.  The bench line labels the figure proxy_ncu_constant.
 PM3_TRAFFIC_PER_BOX = {
-    "deposit_pm3": (15048960 + 707247360) / 64,
-    "fft_z_green_pm3": 1.910046e9 / 64,
-    "fft_c2r_pm3": 1.485638e9 / 64,
+    "deposit_pm3": (23211776 + 707170816) / 64,
+    "fft_x_pm3": (765469696 + 725811456) / 64,
+    "fft_z_green_pm3": (796615936 + 672372224) / 64,
+    "fft_c2r_pm3": (731107584 + 612699904) / 64,
 }
 
 
@@ -484,7 +485,7 @@ def full_run_leg(args, local, rank, nsteps=100):
                                                              stage_first)},
                        "pm3_classes_end": list(so.napm)[2:6], "max_cell_end": int(st[3].max()),
                        "pp_pairs_per_step": pairs // nsteps, "pp_candidates_per_step": cand // nsteps,
-                       "deposit": "int64 fixed-point" if fixed else "fp32 atomics", "graph": fixed,
+                       "deposit": "int64 fixed-point" if fixed else "fp32", "graph": fixed,
                        "pp": "queue" if q.pp_queue else "thread"}
     knyq = math.pi * nw / 1000.0
     b = xis["plain"]
@@ -755,8 +756,8 @@ def main():
                 traffic = int(PM3_TRAFFIC_PER_BOX[dom[1]] * napm[2] / launches_per_step)
             roof = {"kernel": dom[1], "bound": "hbm", "achieved": round(ach, 1), "peak": hbm, "unit": "GB/s",
                     "frac": round(ach / hbm, 4), "traffic": traffic,
-                    "traffic_source": ("proxy_ncu_constant: ncu DRAM bytes of one 64-box launch of the proxy "
-                                       "workload, scaled by boxes (not measured in this run)" if traffic else None),
+                    "traffic_source": ("proxy_ncu_constant: ncu DRAM bytes of one 64-box launch over one tile "
+                                       "of the workload, scaled by boxes (not measured in this run)" if traffic else None),
                     "peak_kind": peak_kind, "avg_launch_ms": round(dom[3], 4),
                     "launches_per_step": launches_per_step,
                     "algorithmic_bytes_per_launch": int(dom[4] / launches_per_step)}
@@ -780,12 +781,12 @@ def main():
             cpu = {"value": round(v, 1), "unit": "particle-steps/s", "cores": cores, "kind": "port",
                    "sample": sample, "sample_seconds": round(secs, 2), "extrapolated_to_full_step": True}
         forms = {"chosen": {"value": round(value, 1), "ms_per_step": round(R["dev_s"] * 1e3 / args.steps, 3),
-                            "deposit": "int64 fixed-point" if fixed else "fp32 atomics",
+                            "deposit": "int64 fixed-point" if fixed else "fp32",
                             "graph": bool(p.step_graph), "pp": "queue" if p.pp_queue else "thread"}}
         precision = None
         if plain:
             forms["plain"] = {"value": round(plain["value"], 1), "ms_per_step": round(plain["ms_per_step"], 3),
-                              "deposit": "fp32 atomics", "graph": False, "pp": "thread",
+                              "deposit": "fp32", "graph": False, "pp": "thread",
                               "stage_ms_per_step": {k: round(float(v), 3) for k, v in
                                                     zip(("drift", "pm1", "pm2", "pm3", "pp", "kick", "step"),
                                                         plain["stage"])}}
@@ -803,7 +804,7 @@ def main():
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "fp32",
             "data": "synthetic (Zel'dovich ICs z=49, EH no-wiggle, seeded)",
             "config": {"workload": desc, "particles_per_gpu": n, "ng": p.ng, "box": p.box,
-                       "deposit": "int64 fixed-point" if fixed else "fp32 atomics",
+                       "deposit": "int64 fixed-point" if fixed else "fp32",
                        "step_graph": bool(p.step_graph), "pp": "queue" if p.pp_queue else "thread",
                        "timestep": "reference adaptive (timestep.f90)", "parallelism": "replicas x%d" % world,
                        "l2": "inputs larger than L2 (%.1f GB particle state)" % (n * 26 / 1e9),

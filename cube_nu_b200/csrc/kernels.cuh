@@ -740,7 +740,8 @@ inline int mass3_groups(int64_t ncells) { return ncells <= (1 << 18) ? 1 : MASS3
 // the write-out reads and clears them without conflicts (side by side, bank conflicts took
 // half of the shared-memory pipe's time, which was 72% busy).  One region of 24^3 cells per block, which looked at 4.6 times
 // its particles and took the whole 27-cell loop in nearly every warp, took 4.64 ms for 512
-// boxes of 144^3 and the PM2 reductions into memory 2.19 ms for eight of 288^3.
+// boxes of 144^3, 3.13 now, and the PM2 reductions into memory 2.19 ms for eight of 288^3,
+// 1.55 now.
 // =================================================================================
 constexpr int DEPB_T = 320, DEPB_SEG = 96;
 constexpr int DEPB_SMEM = 96 * 1024;  // ring of one block: two blocks per SM
